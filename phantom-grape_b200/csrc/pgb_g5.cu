@@ -51,8 +51,9 @@ constexpr int MAXDEV = 64;
 // most of its threads); the table
 // kind keeps its force table in static shared memory (CTAs of <= 256 threads) and the quad
 // kind stages three words per cell (<= 512 threads).  Plans pick one with pgb5_plan_tune.
-// G5C_*J: the j-paired form (newton point masses and quadrupole cells only;
-// pgb_g5_kernels.cuh g5_newton_jpair / g5_quad_jpair).
+// The 64-thread configurations run the slot kernel (pgb_g5_kernels.cuh g5_slots_kernel; 64x1 and
+// 64x1J are the same kernel, and the autotuner times it once).  G5C_256x1J, G5C_1024x1J: the
+// j-paired form of the large CTAs (newton point masses and quadrupole cells only).
 enum G5Cfg {
     G5C_128x4 = 0, G5C_256x2 = 1, G5C_512x2 = 2, G5C_1024x1 = 3, G5C_384x2 = 4, G5C_128x2 = 5, G5C_128x1 = 6,
     G5C_64x1 = 7, G5C_64x1J = 8, G5C_1024x1J = 9, G5C_256x1J = 10, G5_NCFG = 11
@@ -60,7 +61,6 @@ enum G5Cfg {
 constexpr int G5C_NT[G5_NCFG] = {128, 256, 512, 1024, 384, 128, 128, 64, 64, 1024, 256};
 constexpr int G5C_IPT[G5_NCFG] = {4, 2, 2, 1, 2, 2, 1, 1, 1, 1, 1};
 inline bool cfg_jp(int c) { return c >= G5C_64x1J; }
-constexpr int ITILE_MAX = 1024;
 inline int cfg_itile(int c) { return G5C_NT[c] * G5C_IPT[c]; }
 template <int KIND, int NT>
 constexpr bool kind_fits() {
@@ -120,8 +120,13 @@ cudaError_t launch_k(int grid, const G5Args& a, cudaStream_t s, int* occ) {
     } else {
         // the table kind's table lives in dynamic shared memory (a.tbl_size entries)
         const size_t dyn = (KIND == G5_TABLE) ? (size_t)a.tbl_size * sizeof(float2) : 0;
-        if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, g5_kernel<KIND, NT, IPT, JP>, NT, dyn);
-        g5_kernel<KIND, NT, IPT, JP><<<grid, NT, dyn, s>>>(a);
+        // the 64-thread configurations run the slot kernel
+        auto kern = []() {
+            if constexpr (NT == G5S_NT) return g5_slots_kernel<KIND>;
+            else return g5_kernel<KIND, NT, IPT, JP>;
+        }();
+        if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, NT, dyn);
+        kern<<<grid, NT, dyn, s>>>(a);
         return cudaGetLastError();
     }
 }
@@ -178,14 +183,18 @@ int occupancy_of(int kind, int cfg) {
 }
 
 // Default configuration of a call or plan whose largest item has ni i-particles (and
-// PGB_G5_CFG forces one for sweeps): big CTAs for big items, 256-particle tiles for groups.
+// PGB_G5_CFG forces one for sweeps): the slot kernel (64x1), which keeps its rate down to tasks of
+// a few i and fills the GPU with small tasks; only a large direct sum of point masses gains from
+// the larger tasks of the 1024-thread j-paired CTAs.  Measured (us, 64x1 / 1024x1J / the 128x2,
+// 256x2 or 1024x1 scalar form that was the default): newton 999^2 10.5 / 21.6 / 18.7, 256 x 20000
+// 26.5 / 37.2 / 98.8, 4096^2 21.7 / 35.1 / 35.3, 8000^2 46.0 / 47.5 / 51.5, 16384^2 146 / 133 / 148,
+// 65536^2 2022 / 1914 / 2162; a tree of 2^16 particles 55 (points) and 195 (cells) against 370 and
+// 1636 with 128x2, 310-particle TreePM groups 2282 against 5319 with 256x2.
+constexpr long long G5_LARGE_NI = 12288;
 int pick_cfg(int kind, long long ni_max) {
     static int forced = env_int("PGB_G5_CFG", -1, -1, G5_NCFG - 1);
     if (forced >= 0 && cfg_valid(kind, forced)) return forced;
-    if (kind == G5_TABLE || kind == G5_QUAD) return ni_max <= 256 ? G5C_128x2 : G5C_256x2;
-    if (ni_max <= 256) return G5C_128x2;
-    if (ni_max <= 2048) return G5C_256x2;
-    return G5C_1024x1;
+    return kind == G5_NEWTON && ni_max > G5_LARGE_NI ? G5C_1024x1J : G5C_64x1;
 }
 
 // Chunk length for one item: its tasks are all the same size, so one wave of tasks (one per
@@ -324,9 +333,9 @@ inline float scale_i(double x) {
 struct Launcher {
     Stager<float4, double4> st;
 
-    bool stage(cudaStream_t s, const std::vector<Task>& tasks, const std::vector<Group>& groups, int rows,
+    bool stage(cudaStream_t s, const std::vector<Task>& tasks, const std::vector<Group>& groups, int rows, int itile,
                const float4* i_host, int ni_host) {
-        PGB_CUDA_OR(g_err, LIB, st.stage(s, tasks, groups, rows, ITILE_MAX, i_host, ni_host), return false);
+        PGB_CUDA_OR(g_err, LIB, st.stage(s, tasks, groups, rows, itile, i_host, ni_host), return false);
         return true;
     }
 
@@ -523,7 +532,7 @@ bool compute(Dev& d, int kind, int ni, const float4* ih) {
     int rows = plan_item(tasks, groups, 0, ni, 0, nj, itile, jchunk, 0);
     const float4* jpos = kind == G5_QUAD ? d.cd.p : d.jd.p;
     const float4* jaux = kind == G5_QUAD ? d.cqd.p : (kind == G5_SYMMETRIC ? d.jed.p : nullptr);
-    if (!d.L.stage(d.stream, tasks, groups, rows, ih, ni)) return false;
+    if (!d.L.stage(d.stream, tasks, groups, rows, itile, ih, ni)) return false;
     if (!d.L.launch(kind, cfg, d.stream, nullptr, jpos, jaux, d.outd.p)) return false;
     if (ni > 0)
         PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(d.outh.p, d.outd.p, (size_t)ni * sizeof(double4),
@@ -1074,7 +1083,7 @@ void set_tuned(long long key, int cfg) {
 }
 
 bool stage_plan(pgb5_plan* P, cudaStream_t s) {
-    return P->L.stage(s, P->tasks, P->groups, P->rows, nullptr, 0);
+    return P->L.stage(s, P->tasks, P->groups, P->rows, cfg_itile(P->cfg), nullptr, 0);
 }
 }  // namespace
 
@@ -1199,7 +1208,7 @@ int tune_impl(pgb5_plan* P, const void* ipos, const void* jpos, const void* jaux
     int best = P->cfg;
     float best_t = 1e30f;
     for (int cfg = 0; cfg < G5_NCFG; cfg++) {
-        if (!cfg_valid(P->kind, cfg)) continue;
+        if (!cfg_valid(P->kind, cfg) || cfg == G5C_64x1J) continue;   // 64x1J is 64x1
         P->cfg = cfg;
         plan_items(P);
         if (!stage_plan(P, s)) break;

@@ -257,43 +257,47 @@ __device__ __forceinline__ void g5_interact2(const float4* sj, int j, const floa
     }
 }
 
-// ---- j-paired form (the 64-thread tree-code CTAs) ------------------------------------------
+// ---- j-paired forms -------------------------------------------------------------------------
 // One i-particle against two consecutive j records (a "j-pair"), the j-tile held in shared memory
-// as one array per field (G5TileSoA), so that a 16-byte shared load returns a field of four
-// consecutive j and every paired FP32 operand is a natural register pair: (j, j+1) for the j
-// fields, a loop-invariant (v, v) for the i position.  The relative coordinates and the
-// accumulations -- and for cells the Q.dr products and D -- issue as paired FP32 instructions on
-// the heavy half of the FMA pipe, the rest of the chain stays scalar, loading the two halves
-// about equally.  Per pair the arithmetic is g5_interact's, operation for operation (FADD2 /
-// FFMA2 round each lane as FADD / FFMA): the two lanes of an accumulator sum the even and the
-// odd j.
-template <int NT>
-struct G5TileSoA {
-    float x[NT], y[NT], z[NT], m[NT];
-    float q[6][NT];   // cells: G5_QSCALE (q00 q01 q02 q11 q12 q22)
-};
-
+// as one array per field, so that a 16-byte shared load returns a field of four consecutive j and
+// every paired FP32 operand is a natural register pair: (j, j+1) for the j fields, a
+// loop-invariant (v, v) for the i position.  Every FP32 operation issues paired (FADD2 / FMUL2 /
+// FFMA2: two lanes an instruction, each rounded as the scalar one); only the rsqrt, the table
+// look-up and the clamp run per lane.  Per pair the arithmetic is g5_interact's / g5_table_pair's,
+// operation for operation: the two lanes of an accumulator sum the even and the odd j.
 __device__ __forceinline__ void g5_newton_jpair(float2 X, float2 Y, float2 Z, float2 M, float2 nx, float2 ny,
-                                                float2 nz, float e, float2 (&a)[4]) {
+                                                float2 nz, float2 e, float2 (&a)[4]) {
     const float2 dx = __fadd2_rn(X, nx), dy = __fadd2_rn(Y, ny), dz = __fadd2_rn(Z, nz);
-    float2 mq, q;
-    const float* dxp = &dx.x;
-    const float* dyp = &dy.x;
-    const float* dzp = &dz.x;
-    const float* mp = &M.x;
-    float* mqp = &mq.x;
-    float* qp = &q.x;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const float r2 = __fmaf_rn(dzp[h], dzp[h], __fmaf_rn(dyp[h], dyp[h], __fmaf_rn(dxp[h], dxp[h], e)));
-        qp[h] = pair_scale(r2);
-        mqp[h] = mp[h] * qp[h];
-    }
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, e)));
+    const float2 q = make_float2(pair_scale(r2.x), pair_scale(r2.y));
+    const float2 mq = __fmul2_rn(M, q);
     const float2 mq3 = __fmul2_rn(mq, __fmul2_rn(q, q));
     a[3] = __fadd2_rn(a[3], mq);
     a[0] = __ffma2_rn(mq3, dx, a[0]);
     a[1] = __ffma2_rn(mq3, dy, a[1]);
     a[2] = __ffma2_rn(mq3, dz, a[2]);
+}
+
+// The cutoff force (g5_table_pair): `tab` is the shared-memory address of the table less the byte
+// offset of the entry of 2.0, so that the node's bits shifted right by shift - 3 are the entry's
+// byte offset (an entry is 8 bytes).  s - node is formed as node * (-1) + s, which is exact.
+__device__ __forceinline__ void g5_table_jpair(float2 X, float2 Y, float2 Z, float2 M, float2 nx, float2 ny,
+                                               float2 nz, unsigned tab, int shift3, unsigned nodemask, float r2cut,
+                                               float2 (&a)[4]) {
+    const float2 dx = __fadd2_rn(X, nx), dy = __fadd2_rn(Y, ny), dz = __fadd2_rn(Z, nz);
+    float2 s = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, make_float2(2.0f, 2.0f))));
+    s = make_float2(fminf(s.x, r2cut), fminf(s.y, r2cut));
+    const unsigned u0 = __float_as_uint(s.x) & nodemask, u1 = __float_as_uint(s.y) & nodemask;
+    float2 t0, t1;
+    asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(t0.x), "=f"(t0.y) : "r"(tab + (u0 >> shift3)));
+    asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(t1.x), "=f"(t1.y) : "r"(tab + (u1 >> shift3)));
+    const float2 d = __ffma2_rn(make_float2(__uint_as_float(u0), __uint_as_float(u1)), make_float2(-1.0f, -1.0f), s);
+    // per lane: an entry's (f, df/ds) arrive as a register pair, which a paired FMA over the two
+    // entries would first have to be transposed
+    const float2 mf = __fmul2_rn(M, make_float2(__fmaf_rn(d.x, t0.y, t0.x), __fmaf_rn(d.y, t1.y, t1.x)));
+    a[0] = __ffma2_rn(mf, dx, a[0]);
+    a[1] = __ffma2_rn(mf, dy, a[1]);
+    a[2] = __ffma2_rn(mf, dz, a[2]);
 }
 
 // Q = (q00 q01 q02 q11 q12 q22) of the two cells, as pairs, staged as Q' = G5_QSCALE Q: the
@@ -303,13 +307,13 @@ __device__ __forceinline__ void g5_newton_jpair(float2 X, float2 Y, float2 Z, fl
 // instructions per j-pair); pairing them as well (33 paired) follows the Hermite j-paired forms,
 // where the same move made the largest call 5 % faster.
 __device__ __forceinline__ void g5_quad_jpair(float2 X, float2 Y, float2 Z, float2 M, const float2 (&Q)[6], float2 nx,
-                                              float2 ny, float2 nz, float e, float2 (&a)[5]) {
+                                              float2 ny, float2 nz, float2 e, float2 (&a)[5]) {
     const float2 dx = __fadd2_rn(X, nx), dy = __fadd2_rn(Y, ny), dz = __fadd2_rn(Z, nz);
     const float2 vx = __ffma2_rn(Q[2], dz, __ffma2_rn(Q[1], dy, __fmul2_rn(Q[0], dx)));
     const float2 vy = __ffma2_rn(Q[4], dz, __ffma2_rn(Q[3], dy, __fmul2_rn(Q[1], dx)));
     const float2 vz = __ffma2_rn(Q[5], dz, __ffma2_rn(Q[4], dy, __fmul2_rn(Q[2], dx)));
     const float2 D = __ffma2_rn(dz, vz, __ffma2_rn(dy, vy, __fmul2_rn(dx, vx)));
-    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, make_float2(e, e))));
+    const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, e)));
     const float2 q = make_float2(pair_scale(r2.x), pair_scale(r2.y));
     const float2 q2 = __fmul2_rn(q, q), q3 = __fmul2_rn(q2, q), q4 = __fmul2_rn(q2, q2);
     const float2 p = __fmul2_rn(q4, __fmul2_rn(make_float2(G5_QK, G5_QK), q));
@@ -334,34 +338,64 @@ __device__ __forceinline__ double4 add4(double4 a, double4 b) {
     return make_double4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
 }
 
-// One lane's pass over a j tile: records first, first + STRIDE, ... < nt (STRIDE 0: the
-// runtime stride `nl`), accumulated in that order.
-template <int KIND, int NT, int IPT, int STRIDE>
-__device__ __forceinline__ void g5_jloop(const float4* sj, int first, int nt, const float* xi, const float* yi,
-                                         const float* zi, const float* ei, const float2* tab, int shift, float r2cut,
-                                         float (&a)[IPT][NAcc<KIND>::n], int nl = 1) {
-    const int step = STRIDE > 0 ? STRIDE : nl;
-#pragma unroll 4
-    for (int j = first; j < nt; j += step) {
-        if constexpr (KIND == G5_TABLE) {
-            const float4 J = sj[j];
-#pragma unroll
-            for (int k = 0; k < IPT; k++) g5_table_pair(J, xi[k], yi[k], zi[k], tab, shift, r2cut, a[k]);
-        } else {
-#pragma unroll
-            for (int k = 0; k < IPT; k++) g5_interact<KIND, NT>(sj, j, xi[k], yi[k], zi[k], ei[k], a[k]);
+// After a task of a split group: the last CTA to finish one of the group's tasks reduces the
+// group's partial rows (every thread of the CTA calls this).
+template <int KIND, int NT>
+__device__ __forceinline__ void g5_group_done(const G5Args& A, const Task& T, double4* red, int* s_flag) {
+    const Group G = A.groups[T.group];
+    if (group_arrive(A.group_counters, T.group, G.nchunk, s_flag)) {
+        // Cooperative reduction of the group's partial rows: P threads per i, each summing a
+        // fixed strided subset of the rows, then the P sums in thread order (deterministic
+        // for a given group shape).  `red`: NT double4 of shared memory.
+        int P = 1;
+        while (P * 2 * G.ni <= NT) P *= 2;
+        const int per = NT / P;
+        for (int base = 0; base < G.ni; base += per) {
+            const int li = base + threadIdx.x / P, p = threadIdx.x % P;
+            double4 s = make_double4(0, 0, 0, 0);
+            if (li < G.ni) {
+                // four independent partial sums keep four rows' loads in flight; combined in
+                // a fixed order (deterministic)
+                const double4* col = A.partial + (size_t)G.slot0 * A.itile + li;
+                auto ld = [&](int c) {
+                    const double4* r = col + (size_t)c * A.itile;
+                    return make_double4(__ldcg(&r->x), __ldcg(&r->y), __ldcg(&r->z), __ldcg(&r->w));
+                };
+                double4 s1 = s, s2 = s, s3 = s;
+                int c = p;
+                for (; c + 3 * P < G.nchunk; c += 4 * P) {
+                    double4 v0 = ld(c), v1 = ld(c + P), v2 = ld(c + 2 * P), v3 = ld(c + 3 * P);
+                    s = add4(s, v0);
+                    s1 = add4(s1, v1);
+                    s2 = add4(s2, v2);
+                    s3 = add4(s3, v3);
+                }
+                for (; c < G.nchunk; c += P) s = add4(s, ld(c));
+                s = add4(add4(s, s1), add4(s2, s3));
+            }
+            __syncthreads();
+            red[threadIdx.x] = s;
+            __syncthreads();
+            if (p == 0 && li < G.ni) {
+                for (int q = 1; q < P; q++) s = add4(s, red[threadIdx.x + q]);
+                A.out[G.i0 + li] = g5_finish<KIND>(s, A.ascale);
+            }
         }
     }
 }
 
+// The kernel of the CTAs of 128 threads and more: IPT i per thread.  JP: the j-paired form (point
+// masses and cells, one i per thread), else records of one float4 word each (W words).
+template <int NT>
+struct G5TileSoA {
+    float x[NT], y[NT], z[NT], m[NT];
+    float q[6][NT];   // cells: G5_QSCALE (q00 q01 q02 q11 q12 q22)
+};
+
 template <int KIND, int NT, int IPT, bool JP = false>
 __global__ void __launch_bounds__(NT) g5_kernel(G5Args A) {
     constexpr int W = JWords<KIND>::n;   // 16-byte words per j record
-    constexpr bool LANES = (IPT == 1 && NT <= 64);
-    // the j-paired form: newton point masses and quadrupole cells, one i per thread (the
-    // 64-thread CTAs run two for tasks of more than 32 i)
     constexpr bool USE_JP = JP && IPT == 1 && (KIND == G5_NEWTON || KIND == G5_QUAD);
-    constexpr int KM = LANES ? 2 : 1;   // i per thread at most in the j-paired form
     constexpr int SJ_RECS = NT * (W > 2 ? W : 2);
     constexpr int SJ_SOA = USE_JP ? (int)((sizeof(G5TileSoA<NT>) + 15) / 16) : 0;
     __shared__ float4 sj[SJ_RECS > SJ_SOA ? SJ_RECS : SJ_SOA];  // also the reduction buffer (double4 x NT)
@@ -377,312 +411,71 @@ __global__ void __launch_bounds__(NT) g5_kernel(G5Args A) {
         tab = g5_dyn_tab - (0x40000000u >> shift);  // index by (bits of s) >> shift directly
         __syncthreads();
     }
+    const int tid = (int)threadIdx.x;
 
-    // Tasks of more than NT/2 i in the 64-thread one-i-per-thread CTAs: two i per thread
-    // (slot and slot + NT/2) and two j-lanes (even and odd records of each tile), so that every
-    // j record loaded from shared memory serves two i and their sums take paired FP32
-    // instructions; the two lanes' sums are added in lane order.
-    auto lanes_pair_task = [&](const Task& T) {
-        constexpr int H = NT / 2;
-        const int slot = (int)threadIdx.x % H, lane = (int)threadIdx.x / H;
-        float xi[2], yi[2], zi[2], ei[2];
-        double S[2][4];
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int li = slot + k * H;
-            const float4 p = A.ipos[T.i0 + (li < T.ni ? li : 0)];
-            xi[k] = p.x; yi[k] = p.y; zi[k] = p.z; ei[k] = p.w;
-            S[k][0] = S[k][1] = S[k][2] = S[k][3] = 0.0;
-        }
-        for (int jt = 0; jt < T.nj; jt += NT) {
-            const int nt = min(NT, T.nj - jt);
-            __syncthreads();
-            if (threadIdx.x < nt) {
-                const int jk = T.j0 + jt + threadIdx.x;
-                const int jj = A.jidx ? __ldg(A.jidx + jk) : jk;
-                sj[threadIdx.x] = A.jpos[jj];
-                if constexpr (W == 2) sj[NT + threadIdx.x] = A.jaux[jj];
-                if constexpr (W == 3) g5_stage_quad(sj + NT + 2 * threadIdx.x, A.jaux, jj);
-            }
-            __syncthreads();
-            // one block: a lane sees at most NT/2 <= G5_FOLD records of a tile
-            float2 a2[NAcc<KIND>::n];
-#pragma unroll
-            for (int c = 0; c < NAcc<KIND>::n; c++) a2[c] = make_float2(0.f, 0.f);
-#pragma unroll 4
-            for (int j = lane; j < nt; j += 2)
-                g5_interact2<KIND, NT>(sj, j, xi, yi, zi, ei, tab, shift, A.r2cut, a2);
-#pragma unroll
-            for (int k = 0; k < 2; k++) g5_fold2<KIND>(S[k], a2, k);
-        }
-        // lane 1's sums into lane 0's, one i per round through the j-tile buffer
-        double4* red = reinterpret_cast<double4*>(sj);
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            __syncthreads();
-            red[threadIdx.x] = make_double4(S[k][0], S[k][1], S[k][2], S[k][3]);
-            __syncthreads();
-            if (lane == 0) {
-                const double4 v = red[slot + H];
-                S[k][0] += v.x;
-                S[k][1] += v.y;
-                S[k][2] += v.z;
-                S[k][3] += v.w;
-            }
-        }
-        if (lane != 0) return;
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int li = slot + k * H;
-            if (li >= T.ni) continue;
-            const double4 v = make_double4(S[k][0], S[k][1], S[k][2], S[k][3]);
-            if (T.group < 0) A.out[T.i0 + li] = g5_finish<KIND>(v, A.ascale);
-            else A.partial[(size_t)T.slot * A.itile + li] = v;
-        }
-    };
-
-    // Tasks of 33..48 i in the 64-thread CTAs: three i per thread (slot, slot + 16, slot + 32)
-    // over four j-lanes, so that such a task occupies 48 i-slots instead of the pair layout's 64
-    // (tree-code groups of 33..63 i leave a third of those idle); each lane's records are read
-    // once for its three i.  The lanes' sums are added in lane order.
-    auto lanes_triple_task = [&](const Task& T) {
-        constexpr int H = NT / 4;
-        const int slot = (int)threadIdx.x % H, lane = (int)threadIdx.x / H;
-        float xi[3], yi[3], zi[3], ei[3];
-        double S[3][4];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const int li = slot + k * H;
-            const float4 p = A.ipos[T.i0 + (li < T.ni ? li : 0)];
-            xi[k] = p.x; yi[k] = p.y; zi[k] = p.z; ei[k] = p.w;
-            S[k][0] = S[k][1] = S[k][2] = S[k][3] = 0.0;
-        }
-        for (int jt = 0; jt < T.nj; jt += NT) {
-            const int nt = min(NT, T.nj - jt);
-            __syncthreads();
-            if (threadIdx.x < nt) {
-                const int jk = T.j0 + jt + threadIdx.x;
-                const int jj = A.jidx ? __ldg(A.jidx + jk) : jk;
-                sj[threadIdx.x] = A.jpos[jj];
-                if constexpr (W == 2) sj[NT + threadIdx.x] = A.jaux[jj];
-                if constexpr (W == 3) g5_stage_quad(sj + NT + 2 * threadIdx.x, A.jaux, jj);
-            }
-            __syncthreads();
-            // one block: a lane sees at most NT/4 <= G5_FOLD records of a tile
-            float a[3][NAcc<KIND>::n];
-#pragma unroll
-            for (int k = 0; k < 3; k++)
-#pragma unroll
-                for (int c = 0; c < NAcc<KIND>::n; c++) a[k][c] = 0.f;
-            g5_jloop<KIND, NT, 3, 4>(sj, lane, nt, xi, yi, zi, ei, tab, shift, A.r2cut, a);
-#pragma unroll
-            for (int k = 0; k < 3; k++) g5_fold<KIND>(S[k], a[k]);
-        }
-        double4* red = reinterpret_cast<double4*>(sj);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            __syncthreads();
-            red[threadIdx.x] = make_double4(S[k][0], S[k][1], S[k][2], S[k][3]);
-            __syncthreads();
-            if (lane == 0) {
-                for (int l = 1; l < 4; l++) {
-                    const double4 v = red[slot + l * H];
-                    S[k][0] += v.x;
-                    S[k][1] += v.y;
-                    S[k][2] += v.z;
-                    S[k][3] += v.w;
-                }
-            }
-        }
-        if (lane != 0) return;
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            const int li = slot + k * H;
-            if (li >= T.ni) continue;
-            const double4 v = make_double4(S[k][0], S[k][1], S[k][2], S[k][3]);
-            if (T.group < 0) A.out[T.i0 + li] = g5_finish<KIND>(v, A.ascale);
-            else A.partial[(size_t)T.slot * A.itile + li] = v;
-        }
-    };
-
-    // The j-paired task (USE_JP).  In the 64-thread CTAs a task of more than NT/2 i runs two i
-    // per thread (slot and slot + NT/2) over two j-lanes, a smaller one one i per thread over
-    // nl = NT / isl lanes (isl = ni rounded up to 16, as the other form); lane l takes the tile's
-    // j-quads l, l + nl, ...  Larger CTAs: one i per thread, one lane.  The tile is staged as
-    // field arrays padded to a multiple of 4 with massless copies of its first record (and zero
-    // moments for cells), which add exact zeros.  FP32 sums are folded into FP64 every G5_FOLD
-    // j of a lane; the lanes' sums are added in lane order.
-    auto jp_task = [&](const Task& T) {
+    // The j-paired task: one i per thread.  The tile is staged as field arrays padded to a
+    // multiple of 4 with massless copies of its first record (and zero moments for cells), which
+    // add exact zeros.  FP32 sums are folded into FP64 every G5_FOLD j.
+    auto jp_task = [&](const Task& T, double (&S)[4]) {
         G5TileSoA<NT>* sa = reinterpret_cast<G5TileSoA<NT>*>(sj);
-        const bool two = LANES && T.ni > NT / 2;
-        int nl = 1, isl = NT;
-        if (two) {
-            nl = 2;
-            isl = NT / 2;
-        } else if (LANES) {
-            const int need = (T.ni + 15) & ~15;
-            nl = NT / (need > 0 ? need : 32);
-            isl = NT / nl;
-        }
-        const int slot = (int)threadIdx.x % isl, lane = (int)threadIdx.x / isl;
-        const int nik = two ? 2 : 1;
-        float2 nx[KM], ny[KM], nz[KM];
-        float ei[KM];
-        double S[KM][4];
-#pragma unroll
-        for (int k = 0; k < KM; k++) {
-            const int li = slot + k * isl;
-            const float4 p = A.ipos[T.i0 + (li < T.ni ? li : 0)];
-            nx[k] = make_float2(-p.x, -p.x);
-            ny[k] = make_float2(-p.y, -p.y);
-            nz[k] = make_float2(-p.z, -p.z);
-            ei[k] = p.w;
-            S[k][0] = S[k][1] = S[k][2] = S[k][3] = 0.0;
-        }
+        const float4 p = A.ipos[T.i0 + (tid < T.ni ? tid : 0)];
+        const float2 nx = make_float2(-p.x, -p.x), ny = make_float2(-p.y, -p.y), nz = make_float2(-p.z, -p.z);
+        const float2 ei = make_float2(p.w, p.w);
         for (int jt = 0; jt < T.nj; jt += NT) {
             const int nt = min(NT, T.nj - jt);
             const int nt4 = (nt + 3) & ~3;
             __syncthreads();
-            if ((int)threadIdx.x < nt4) {
-                const bool real = (int)threadIdx.x < nt;
-                const int jk = T.j0 + jt + (real ? (int)threadIdx.x : 0);
+            if (tid < nt4) {
+                const bool real = tid < nt;
+                const int jk = T.j0 + jt + (real ? tid : 0);
                 const int jj = A.jidx ? __ldg(A.jidx + jk) : jk;
                 const float4 J = A.jpos[jj];
-                sa->x[threadIdx.x] = J.x;
-                sa->y[threadIdx.x] = J.y;
-                sa->z[threadIdx.x] = J.z;
-                sa->m[threadIdx.x] = real ? J.w : 0.0f;
+                sa->x[tid] = J.x;
+                sa->y[tid] = J.y;
+                sa->z[tid] = J.z;
+                sa->m[tid] = real ? J.w : 0.0f;
                 if constexpr (KIND == G5_QUAD) {
                     const float4 Q0 = A.jaux[2 * jj], Q1 = A.jaux[2 * jj + 1];
                     const float f = real ? G5_QSCALE : 0.0f;
-                    sa->q[0][threadIdx.x] = f * Q0.x;
-                    sa->q[1][threadIdx.x] = f * Q0.y;
-                    sa->q[2][threadIdx.x] = f * Q0.z;
-                    sa->q[3][threadIdx.x] = f * Q0.w;
-                    sa->q[4][threadIdx.x] = f * Q1.x;
-                    sa->q[5][threadIdx.x] = f * Q1.y;
+                    sa->q[0][tid] = f * Q0.x;
+                    sa->q[1][tid] = f * Q0.y;
+                    sa->q[2][tid] = f * Q0.z;
+                    sa->q[3][tid] = f * Q0.w;
+                    sa->q[4][tid] = f * Q1.x;
+                    sa->q[5][tid] = f * Q1.y;
                 }
             }
             __syncthreads();
-            for (int jb = 0; jb < nt4; jb += G5_FOLD * nl) {
-            const int je = min(jb + G5_FOLD * nl, nt4);
-            float2 a2[KM][NAcc<KIND>::n];
+            for (int jb = 0; jb < nt4; jb += G5_FOLD) {
+                const int je = min(jb + G5_FOLD, nt4);
+                float2 a2[NAcc<KIND>::n];
 #pragma unroll
-            for (int k = 0; k < KM; k++)
+                for (int c = 0; c < NAcc<KIND>::n; c++) a2[c] = make_float2(0.f, 0.f);
+                for (int j = jb; j < je; j += 4) {
+                    const float4 X = *reinterpret_cast<const float4*>(&sa->x[j]);
+                    const float4 Y = *reinterpret_cast<const float4*>(&sa->y[j]);
+                    const float4 Z = *reinterpret_cast<const float4*>(&sa->z[j]);
+                    const float4 M = *reinterpret_cast<const float4*>(&sa->m[j]);
+                    const float2 xa = make_float2(X.x, X.y), xb = make_float2(X.z, X.w);
+                    const float2 ya = make_float2(Y.x, Y.y), yb = make_float2(Y.z, Y.w);
+                    const float2 za = make_float2(Z.x, Z.y), zb = make_float2(Z.z, Z.w);
+                    const float2 ma = make_float2(M.x, M.y), mb = make_float2(M.z, M.w);
+                    if constexpr (KIND == G5_QUAD) {
+                        float2 Qa[6], Qb[6];
 #pragma unroll
-                for (int c = 0; c < NAcc<KIND>::n; c++) a2[k][c] = make_float2(0.f, 0.f);
-            for (int j = jb + 4 * lane; j < je; j += 4 * nl) {
-                const float4 X = *reinterpret_cast<const float4*>(&sa->x[j]);
-                const float4 Y = *reinterpret_cast<const float4*>(&sa->y[j]);
-                const float4 Z = *reinterpret_cast<const float4*>(&sa->z[j]);
-                const float4 M = *reinterpret_cast<const float4*>(&sa->m[j]);
-                if constexpr (KIND == G5_QUAD) {
-                    float4 Qv[6];
-#pragma unroll
-                    for (int c = 0; c < 6; c++) Qv[c] = *reinterpret_cast<const float4*>(&sa->q[c][j]);
-                    float2 Qa[6], Qb[6];
-#pragma unroll
-                    for (int c = 0; c < 6; c++) {
-                        Qa[c] = make_float2(Qv[c].x, Qv[c].y);
-                        Qb[c] = make_float2(Qv[c].z, Qv[c].w);
-                    }
-#pragma unroll
-                    for (int k = 0; k < KM; k++) {
-                        if (k < nik) {
-                            g5_quad_jpair(make_float2(X.x, X.y), make_float2(Y.x, Y.y), make_float2(Z.x, Z.y),
-                                          make_float2(M.x, M.y), Qa, nx[k], ny[k], nz[k], ei[k], a2[k]);
-                            g5_quad_jpair(make_float2(X.z, X.w), make_float2(Y.z, Y.w), make_float2(Z.z, Z.w),
-                                          make_float2(M.z, M.w), Qb, nx[k], ny[k], nz[k], ei[k], a2[k]);
+                        for (int c = 0; c < 6; c++) {
+                            const float4 v = *reinterpret_cast<const float4*>(&sa->q[c][j]);
+                            Qa[c] = make_float2(v.x, v.y);
+                            Qb[c] = make_float2(v.z, v.w);
                         }
-                    }
-                } else {
-#pragma unroll
-                    for (int k = 0; k < KM; k++) {
-                        if (k < nik) {
-                            g5_newton_jpair(make_float2(X.x, X.y), make_float2(Y.x, Y.y), make_float2(Z.x, Z.y),
-                                            make_float2(M.x, M.y), nx[k], ny[k], nz[k], ei[k], a2[k]);
-                            g5_newton_jpair(make_float2(X.z, X.w), make_float2(Y.z, Y.w), make_float2(Z.z, Z.w),
-                                            make_float2(M.z, M.w), nx[k], ny[k], nz[k], ei[k], a2[k]);
-                        }
+                        g5_quad_jpair(xa, ya, za, ma, Qa, nx, ny, nz, ei, a2);
+                        g5_quad_jpair(xb, yb, zb, mb, Qb, nx, ny, nz, ei, a2);
+                    } else {
+                        g5_newton_jpair(xa, ya, za, ma, nx, ny, nz, ei, a2);
+                        g5_newton_jpair(xb, yb, zb, mb, nx, ny, nz, ei, a2);
                     }
                 }
-            }
-#pragma unroll
-            for (int k = 0; k < KM; k++) g5_fold2<KIND>(S[k], a2[k], -1);
-            }
-        }
-        // lane sums in lane order, one i per round through the j-tile buffer
-        double4* red = reinterpret_cast<double4*>(sj);
-#pragma unroll
-        for (int k = 0; k < KM; k++) {
-            if (k < nik && nl > 1) {
-                __syncthreads();
-                red[threadIdx.x] = make_double4(S[k][0], S[k][1], S[k][2], S[k][3]);
-                __syncthreads();
-                if (lane == 0) {
-                    for (int l = 1; l < nl; l++) {
-                        const double4 v = red[slot + l * isl];
-                        S[k][0] += v.x;
-                        S[k][1] += v.y;
-                        S[k][2] += v.z;
-                        S[k][3] += v.w;
-                    }
-                }
-            }
-        }
-        if (lane != 0) return;
-#pragma unroll
-        for (int k = 0; k < KM; k++) {
-            const int li = slot + k * isl;
-            if (k >= nik || li >= T.ni) continue;
-            const double4 v = make_double4(S[k][0], S[k][1], S[k][2], S[k][3]);
-            if (T.group < 0) A.out[T.i0 + li] = g5_finish<KIND>(v, A.ascale);
-            else A.partial[(size_t)T.slot * A.itile + li] = v;
-        }
-    };
-
-    // The last CTA to finish a task of a split group reduces the group's partial rows.
-    auto group_done = [&](const Task& T) {
-        const Group G = A.groups[T.group];
-        if (group_arrive(A.group_counters, T.group, G.nchunk, &s_flag)) {
-            // Cooperative reduction of the group's partial rows: P threads per i, each summing a
-            // fixed strided subset of the rows, then the P sums in thread order (deterministic
-            // for a given group shape).  `red` reuses the j-tile buffer.
-            double4* red = reinterpret_cast<double4*>(sj);
-            static_assert(sizeof(float4) * NT * (W > 2 ? W : 2) >= sizeof(double4) * NT, "reduction buffer");
-            int P = 1;
-            while (P * 2 * G.ni <= NT) P *= 2;
-            const int per = NT / P;
-            for (int base = 0; base < G.ni; base += per) {
-                const int li = base + threadIdx.x / P, p = threadIdx.x % P;
-                double4 s = make_double4(0, 0, 0, 0);
-                if (li < G.ni) {
-                    // four independent partial sums keep four rows' loads in flight; combined in
-                    // a fixed order (deterministic)
-                    const double4* col = A.partial + (size_t)G.slot0 * A.itile + li;
-                    auto ld = [&](int c) {
-                        const double4* r = col + (size_t)c * A.itile;
-                        return make_double4(__ldcg(&r->x), __ldcg(&r->y), __ldcg(&r->z), __ldcg(&r->w));
-                    };
-                    double4 s1 = s, s2 = s, s3 = s;
-                    int c = p;
-                    for (; c + 3 * P < G.nchunk; c += 4 * P) {
-                        double4 v0 = ld(c), v1 = ld(c + P), v2 = ld(c + 2 * P), v3 = ld(c + 3 * P);
-                        s = add4(s, v0);
-                        s1 = add4(s1, v1);
-                        s2 = add4(s2, v2);
-                        s3 = add4(s3, v3);
-                    }
-                    for (; c < G.nchunk; c += P) s = add4(s, ld(c));
-                    s = add4(add4(s, s1), add4(s2, s3));
-                }
-                __syncthreads();
-                red[threadIdx.x] = s;
-                __syncthreads();
-                if (p == 0 && li < G.ni) {
-                    for (int q = 1; q < P; q++) s = add4(s, red[threadIdx.x + q]);
-                    A.out[G.i0 + li] = g5_finish<KIND>(s, A.ascale);
-                }
+                g5_fold2<KIND>(S, a2, -1);
             }
         }
     };
@@ -691,139 +484,271 @@ __global__ void __launch_bounds__(NT) g5_kernel(G5Args A) {
         int t = next_task(A.task_counter, &s_task, A.ntasks, first);
         if (t >= A.ntasks) break;
         const Task T = A.tasks[t];
-        if constexpr (USE_JP) {
-            jp_task(T);
-            if (T.group >= 0) group_done(T);
-            continue;
-        }
-        if constexpr (LANES) {
-            if (NT == 64 && T.ni > NT / 2 && T.ni <= 3 * NT / 4) {
-                lanes_triple_task(T);
-                if (T.group >= 0) group_done(T);
-                continue;
-            }
-            if (T.ni > NT / 2) {
-                lanes_pair_task(T);
-                if (T.group >= 0) group_done(T);
-                continue;
-            }
-        }
-        // j-lanes (the 64-thread one-i-per-thread CTAs): a task of few i takes half-warps of
-        // i-slots (isl = ni rounded up to 16; the two half-warps of a warp then read two j records,
-        // which a 16-byte shared load serves in the same two wavefronts as a broadcast) and
-        // splits each j-tile over the nl = NT / isl lanes of slots; the lanes' sums are added in
-        // lane order at the end.  Large tasks: nl = 1.
-        int nl = 1, isl = NT;
-        if constexpr (LANES) {
-            const int need = (T.ni + 15) & ~15;
-            nl = NT / (need > 0 ? need : 32);
-            isl = NT / nl;
-        }
-        const int slot = LANES ? (int)threadIdx.x % isl : (int)threadIdx.x;
-        const int lane = LANES ? (int)threadIdx.x / isl : 0;
-
-        float xi[IPT], yi[IPT], zi[IPT], ei[IPT];
         double S[IPT][4];
 #pragma unroll
-        for (int k = 0; k < IPT; k++) {
-            int li = slot + k * NT;
-            int ii = T.i0 + (li < T.ni ? li : 0);
-            float4 p = A.ipos[ii];
-            xi[k] = p.x; yi[k] = p.y; zi[k] = p.z; ei[k] = p.w;
-            S[k][0] = S[k][1] = S[k][2] = S[k][3] = 0.0;
-        }
-
-        for (int jt = 0; jt < T.nj; jt += NT) {
-            const int nt = min(NT, T.nj - jt);
-            __syncthreads();
-            if (threadIdx.x < nt) {
-                const int jk = T.j0 + jt + threadIdx.x;
-                const int jj = A.jidx ? __ldg(A.jidx + jk) : jk;
-                sj[threadIdx.x] = A.jpos[jj];
-                if constexpr (W == 2) sj[NT + threadIdx.x] = A.jaux[jj];
-                if constexpr (W == 3) g5_stage_quad(sj + NT + 2 * threadIdx.x, A.jaux, jj);
-            }
-            __syncthreads();
-            if constexpr (IPT % 2 == 0) {
-                for (int j0 = 0; j0 < nt; j0 += G5_FOLD) {
-                    const int j1 = min(j0 + G5_FOLD, nt);
-                    float2 a2[IPT / 2][NAcc<KIND>::n];
-#pragma unroll
-                    for (int p = 0; p < IPT / 2; p++)
-#pragma unroll
-                        for (int c = 0; c < NAcc<KIND>::n; c++) a2[p][c] = make_float2(0.f, 0.f);
-#pragma unroll 4
-                    for (int j = j0; j < j1; j++) {
-#pragma unroll
-                        for (int p = 0; p < IPT / 2; p++)
-                            g5_interact2<KIND, NT>(sj, j, xi + 2 * p, yi + 2 * p, zi + 2 * p, ei + 2 * p, tab, shift,
-                                                   A.r2cut, a2[p]);
-                    }
-#pragma unroll
-                    for (int k = 0; k < IPT; k++) g5_fold2<KIND>(S[k], a2[k / 2], k % 2);
-                }
-            } else {
-            // blocks of G5_FOLD terms per lane (one block when a tile has no more: NT <= G5_FOLD);
-            // the lane stride as a template constant, so that the unrolled loop addresses its j
-            // records with immediate offsets (64-thread CTAs have 1, 2 or 4 lanes)
-            const int nlanes = LANES ? nl : 1;
-            auto block = [&](int j0, int j1) {
-                float a[IPT][NAcc<KIND>::n];
-#pragma unroll
-                for (int k = 0; k < IPT; k++)
-#pragma unroll
-                    for (int c = 0; c < NAcc<KIND>::n; c++) a[k][c] = 0.f;
-                if (nlanes == 1) g5_jloop<KIND, NT, IPT, 1>(sj, j0 + lane, j1, xi, yi, zi, ei, tab, shift, A.r2cut, a);
-                else if (nlanes == 2) g5_jloop<KIND, NT, IPT, 2>(sj, j0 + lane, j1, xi, yi, zi, ei, tab, shift, A.r2cut, a);
-                else if (nlanes == 4) g5_jloop<KIND, NT, IPT, 4>(sj, j0 + lane, j1, xi, yi, zi, ei, tab, shift, A.r2cut, a);
-                else g5_jloop<KIND, NT, IPT, 0>(sj, j0 + lane, j1, xi, yi, zi, ei, tab, shift, A.r2cut, a, nlanes);
-#pragma unroll
-                for (int k = 0; k < IPT; k++) g5_fold<KIND>(S[k], a[k]);
-            };
-            if constexpr (NT <= G5_FOLD) {
-                block(0, nt);
-            } else {
-                for (int j0 = 0; j0 < nt; j0 += G5_FOLD * nlanes) block(j0, min(j0 + G5_FOLD * nlanes, nt));
-            }
-            }
-        }
-
-        bool lane0 = true;
-        if constexpr (LANES) {
-            if (nl > 1) {
-                // lane sums in lane order through the j-tile buffer (IPT == 1)
-                double4* red = reinterpret_cast<double4*>(sj);
-                __syncthreads();
-                red[threadIdx.x] = make_double4(S[0][0], S[0][1], S[0][2], S[0][3]);
-                __syncthreads();
-                lane0 = lane == 0;
-                if (lane0) {
-                    for (int l = 1; l < nl; l++) {
-                        const double4 v = red[slot + l * isl];
-                        S[0][0] += v.x;
-                        S[0][1] += v.y;
-                        S[0][2] += v.z;
-                        S[0][3] += v.w;
-                    }
-                }
-            }
-        }
-        if (T.group < 0) {
+        for (int k = 0; k < IPT; k++) S[k][0] = S[k][1] = S[k][2] = S[k][3] = 0.0;
+        if constexpr (USE_JP) {
+            jp_task(T, S[0]);
+        } else {
+            float xi[IPT], yi[IPT], zi[IPT], ei[IPT];
 #pragma unroll
             for (int k = 0; k < IPT; k++) {
-                int li = slot + k * NT;
-                if (lane0 && li < T.ni)
-                    A.out[T.i0 + li] = g5_finish<KIND>(make_double4(S[k][0], S[k][1], S[k][2], S[k][3]), A.ascale);
+                int li = tid + k * NT;
+                int ii = T.i0 + (li < T.ni ? li : 0);
+                float4 p = A.ipos[ii];
+                xi[k] = p.x; yi[k] = p.y; zi[k] = p.z; ei[k] = p.w;
             }
-            continue;
+            for (int jt = 0; jt < T.nj; jt += NT) {
+                const int nt = min(NT, T.nj - jt);
+                __syncthreads();
+                if (tid < nt) {
+                    const int jk = T.j0 + jt + tid;
+                    const int jj = A.jidx ? __ldg(A.jidx + jk) : jk;
+                    sj[tid] = A.jpos[jj];
+                    if constexpr (W == 2) sj[NT + tid] = A.jaux[jj];
+                    if constexpr (W == 3) g5_stage_quad(sj + NT + 2 * tid, A.jaux, jj);
+                }
+                __syncthreads();
+                for (int j0 = 0; j0 < nt; j0 += G5_FOLD) {
+                    const int j1 = min(j0 + G5_FOLD, nt);
+                    if constexpr (IPT % 2 == 0) {
+                        float2 a2[IPT / 2][NAcc<KIND>::n];
+#pragma unroll
+                        for (int p = 0; p < IPT / 2; p++)
+#pragma unroll
+                            for (int c = 0; c < NAcc<KIND>::n; c++) a2[p][c] = make_float2(0.f, 0.f);
+#pragma unroll 4
+                        for (int j = j0; j < j1; j++) {
+#pragma unroll
+                            for (int p = 0; p < IPT / 2; p++)
+                                g5_interact2<KIND, NT>(sj, j, xi + 2 * p, yi + 2 * p, zi + 2 * p, ei + 2 * p, tab, shift,
+                                                       A.r2cut, a2[p]);
+                        }
+#pragma unroll
+                        for (int k = 0; k < IPT; k++) g5_fold2<KIND>(S[k], a2[k / 2], k % 2);
+                    } else {
+                        float a[IPT][NAcc<KIND>::n];
+#pragma unroll
+                        for (int k = 0; k < IPT; k++)
+#pragma unroll
+                            for (int c = 0; c < NAcc<KIND>::n; c++) a[k][c] = 0.f;
+#pragma unroll 4
+                        for (int j = j0; j < j1; j++) {
+#pragma unroll
+                            for (int k = 0; k < IPT; k++) {
+                                if constexpr (KIND == G5_TABLE)
+                                    g5_table_pair(sj[j], xi[k], yi[k], zi[k], tab, shift, A.r2cut, a[k]);
+                                else
+                                    g5_interact<KIND, NT>(sj, j, xi[k], yi[k], zi[k], ei[k], a[k]);
+                            }
+                        }
+#pragma unroll
+                        for (int k = 0; k < IPT; k++) g5_fold<KIND>(S[k], a[k]);
+                    }
+                }
+            }
         }
-        double4* row = A.partial + (size_t)T.slot * A.itile;
 #pragma unroll
         for (int k = 0; k < IPT; k++) {
-            int li = slot + k * NT;
-            if (lane0 && li < T.ni) row[li] = make_double4(S[k][0], S[k][1], S[k][2], S[k][3]);
+            const int li = tid + k * NT;
+            if (li >= T.ni) continue;
+            const double4 v = make_double4(S[k][0], S[k][1], S[k][2], S[k][3]);
+            if (T.group < 0) A.out[T.i0 + li] = g5_finish<KIND>(v, A.ascale);
+            else A.partial[(size_t)T.slot * A.itile + li] = v;
         }
-        group_done(T);
+        if (T.group >= 0) g5_group_done<KIND, NT>(A, T, reinterpret_cast<double4*>(sj), &s_flag);
+    }
+}
+
+// ---- the 64-thread kernel: i-slots x j-lanes ------------------------------------------------
+// Every task of a 64-thread CTA runs as 16 i-slots over four j-lanes, IPT = ceil(ni / 16) i per
+// thread (slot, slot + 16, ...), j-paired.  It is built for batches of small, uneven groups (tree
+// and TreePM groups of a few tens to a few hundred i), which the FMA pipe bounds:
+//  * a task leaves at most 15 of its slots idle, whatever its size (a 75-particle group runs as
+//    64 + 11: 80 slots; 9.6 % of the slots of an N = 2^20 tree's cell pairs are idle);
+//  * the j records read from shared memory serve IPT i: a full task reads a 16-byte word per 4
+//    pairs (point masses) or 1.6 pairs (cells);
+//  * every FP32 operation is paired: a cell pair takes 16.5 + 1 (rsqrt) instructions instead of 34.
+// Against the one-record-per-load form it replaces (one to three i per thread, two to four lanes,
+// scalar chains): cells of an N = 2^20 tree 4156 -> 3563 us (799 Gint/s: with the idle slots 79 %
+// of the FMA rate), its point masses 974 -> 831 us (1930 Gint/s), the 4096 TreePM groups of 2^20
+// particles 2906 -> 2282 us (1955 Gint/s; 12 FMA operations, 4 integer ones and a table look-up of
+// 2.2 shared wavefronts a pair: FMA heavy half 70 %, shared wavefronts 60 %, issue 62 % busy).
+// A j-tile is G5S_NJ records as field arrays; lane l takes the tile's j-quads l, l + 4, ....  The
+// tile is padded to a multiple of 4 with massless records far away (G5S_FAR), which add exact
+// zeros to any finite sum.  FP32 sums cover a tile (32 terms a lane half and i at most), then go
+// into the FP64 sums; the lanes' sums are added in lane order at the end of the task.
+constexpr int G5S_NT = 64, G5S_SLOTS = 16, G5S_LANES = 4, G5S_IPT = 4;
+constexpr int G5S_NJ = 256;   // records a tile: 64 a lane between two folds into FP64 (128: cells 3 % slower)
+// Resident CTAs asked of the compiler: cells 5 (167 registers, 10 warps an SM: 3563 us; 8 CTAs of 128
+// registers, which reload the j fields per pair, 3639), point masses and the table 10 (95 registers)
+template <int KIND>
+constexpr int g5s_min_ctas() { return KIND == G5_QUAD ? 5 : 10; }
+constexpr float G5S_FAR = 1e18f;   // its square times three is finite
+
+template <int KIND>
+struct G5STile {
+    static constexpr int NQ = KIND == G5_QUAD ? 6 : (KIND == G5_SYMMETRIC ? 1 : 0);   // extra fields
+    float f[4 + NQ][G5S_NJ];   // x y z m, then the moments (G5_QSCALE q00 q01 q02 q11 q12 q22) or eps2_j
+};
+
+template <int KIND>
+struct G5SShared {
+    G5STile<KIND> t;
+    double S[G5S_IPT][4][G5S_NT];   // the FP64 sums: i k, component c of thread t at S[k][c][t]
+};
+
+template <int KIND, int IPT>
+__device__ __forceinline__ void g5_slots_task(const G5Args& A, const Task& T, G5SShared<KIND>& sh, unsigned tab) {
+    constexpr int NJ = G5S_NJ, R = NJ / G5S_NT;
+    constexpr int NC = KIND == G5_TABLE ? 3 : 4;   // components that are summed
+    const int tid = (int)threadIdx.x, slot = tid % G5S_SLOTS, lane = tid / G5S_SLOTS;
+    float2 nx[IPT], ny[IPT], nz[IPT], ei[IPT];
+#pragma unroll
+    for (int k = 0; k < IPT; k++) {
+        const int li = slot + k * G5S_SLOTS;
+        const float4 p = A.ipos[T.i0 + (li < T.ni ? li : 0)];
+        nx[k] = make_float2(-p.x, -p.x);
+        ny[k] = make_float2(-p.y, -p.y);
+        nz[k] = make_float2(-p.z, -p.z);
+        ei[k] = make_float2(p.w, p.w);
+#pragma unroll
+        for (int c = 0; c < 4; c++) sh.S[k][c][tid] = 0.0;
+    }
+    const int shift3 = A.tbl_shift - 3;
+    const unsigned nodemask = ~0u << (A.tbl_shift & 31);
+    int jn[R];
+    auto load_idx = [&](int j0) {
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int q = j0 + tid + r * G5S_NT;
+            jn[r] = T.j0 + q;
+            if (A.jidx && q < T.nj) jn[r] = __ldg(A.jidx + T.j0 + q);
+        }
+    };
+    load_idx(0);
+    for (int jt = 0; jt < T.nj; jt += NJ) {
+        const int nt = min(NJ, T.nj - jt), nq = (nt + 3) >> 2;
+        float4 J[R];
+        float4 Q0[R], Q1[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int q = tid + r * G5S_NT;
+            J[r] = make_float4(G5S_FAR, G5S_FAR, G5S_FAR, 0.f);
+            Q0[r] = Q1[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (q < nt) {
+                const int jj = jn[r];
+                J[r] = A.jpos[jj];
+                if constexpr (KIND == G5_QUAD) {
+                    Q0[r] = scale4(A.jaux[2 * (size_t)jj], G5_QSCALE);
+                    Q1[r] = scale4(A.jaux[2 * (size_t)jj + 1], G5_QSCALE);
+                }
+                if constexpr (KIND == G5_SYMMETRIC) Q0[r].x = A.jaux[jj].x;
+            }
+        }
+        __syncthreads();   // the tile before has been read
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            const int q = tid + r * G5S_NT;
+            if (q < 4 * nq) {
+                float(*f)[NJ] = sh.t.f;
+                f[0][q] = J[r].x;
+                f[1][q] = J[r].y;
+                f[2][q] = J[r].z;
+                f[3][q] = J[r].w;
+                if constexpr (KIND == G5_QUAD) {
+                    f[4][q] = Q0[r].x;
+                    f[5][q] = Q0[r].y;
+                    f[6][q] = Q0[r].z;
+                    f[7][q] = Q0[r].w;
+                    f[8][q] = Q1[r].x;
+                    f[9][q] = Q1[r].y;
+                }
+                if constexpr (KIND == G5_SYMMETRIC) f[4][q] = Q0[r].x;
+            }
+        }
+        __syncthreads();
+        load_idx(jt + NJ);   // the next tile's indices: its records are then one load away
+        float2 a[IPT][NAcc<KIND>::n];
+#pragma unroll
+        for (int k = 0; k < IPT; k++)
+#pragma unroll
+            for (int c = 0; c < NAcc<KIND>::n; c++) a[k][c] = make_float2(0.f, 0.f);
+#pragma unroll 1
+        for (int jq = lane; jq < nq; jq += G5S_LANES) {
+            float4 v[4 + G5STile<KIND>::NQ];
+#pragma unroll
+            for (int c = 0; c < 4 + G5STile<KIND>::NQ; c++) v[c] = *reinterpret_cast<const float4*>(&sh.t.f[c][4 * jq]);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                float2 w[4 + G5STile<KIND>::NQ];
+#pragma unroll
+                for (int c = 0; c < 4 + G5STile<KIND>::NQ; c++)
+                    w[c] = h ? make_float2(v[c].z, v[c].w) : make_float2(v[c].x, v[c].y);
+#pragma unroll
+                for (int k = 0; k < IPT; k++) {
+                    if constexpr (KIND == G5_QUAD) {
+                        const float2 q[6] = {w[4], w[5], w[6], w[7], w[8], w[9]};
+                        g5_quad_jpair(w[0], w[1], w[2], w[3], q, nx[k], ny[k], nz[k], ei[k], a[k]);
+                    } else if constexpr (KIND == G5_TABLE) {
+                        g5_table_jpair(w[0], w[1], w[2], w[3], nx[k], ny[k], nz[k], tab, shift3, nodemask, A.r2cut, a[k]);
+                    } else if constexpr (KIND == G5_SYMMETRIC) {
+                        g5_newton_jpair(w[0], w[1], w[2], w[3], nx[k], ny[k], nz[k], __fadd2_rn(ei[k], w[4]), a[k]);
+                    } else {
+                        g5_newton_jpair(w[0], w[1], w[2], w[3], nx[k], ny[k], nz[k], ei[k], a[k]);
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < IPT; k++) {
+            double S[4];
+#pragma unroll
+            for (int c = 0; c < NC; c++) S[c] = sh.S[k][c][tid];
+            S[3] = NC > 3 ? S[3] : 0.0;
+            g5_fold2<KIND>(S, a[k], -1);
+#pragma unroll
+            for (int c = 0; c < NC; c++) sh.S[k][c][tid] = S[c];
+        }
+    }
+    // the lanes' sums in lane order: thread t sums i-particle t
+    __syncthreads();
+    if (tid < T.ni) {
+        const int k = tid / G5S_SLOTS, s0 = tid % G5S_SLOTS;
+        double S[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            S[c] = sh.S[k][c][s0];
+#pragma unroll
+            for (int l = 1; l < G5S_LANES; l++) S[c] += sh.S[k][c][s0 + l * G5S_SLOTS];
+        }
+        const double4 v = make_double4(S[0], S[1], S[2], S[3]);
+        if (T.group < 0) A.out[T.i0 + tid] = g5_finish<KIND>(v, A.ascale);
+        else A.partial[(size_t)T.slot * A.itile + tid] = v;
+    }
+    __syncthreads();   // before the sums' or the tile's memory is used again
+}
+
+template <int KIND>
+__global__ void __launch_bounds__(G5S_NT, g5s_min_ctas<KIND>()) g5_slots_kernel(G5Args A) {
+    __shared__ __align__(16) G5SShared<KIND> sh;
+    __shared__ int s_task, s_flag;
+    extern __shared__ float2 g5_dyn_tab[];   // the table kind's force table, for the CTA's lifetime
+    unsigned tab = 0;
+    if constexpr (KIND == G5_TABLE) {
+        for (int k = threadIdx.x; k < A.tbl_size; k += G5S_NT) g5_dyn_tab[k] = A.table[k];
+        tab = (unsigned)__cvta_generic_to_shared(g5_dyn_tab) - (0x40000000u >> (A.tbl_shift - 3));
+        __syncthreads();
+    }
+    for (bool first = true;; first = false) {
+        const int t = next_task(A.task_counter, &s_task, A.ntasks, first);
+        if (t >= A.ntasks) break;
+        const Task T = A.tasks[t];
+        if (T.ni > 3 * G5S_SLOTS) g5_slots_task<KIND, 4>(A, T, sh, tab);
+        else if (T.ni > 2 * G5S_SLOTS) g5_slots_task<KIND, 3>(A, T, sh, tab);
+        else if (T.ni > G5S_SLOTS) g5_slots_task<KIND, 2>(A, T, sh, tab);
+        else g5_slots_task<KIND, 1>(A, T, sh, tab);
+        if (T.group >= 0) g5_group_done<KIND, G5S_NT>(A, T, reinterpret_cast<double4*>(&sh), &s_flag);
     }
 }
 
