@@ -933,9 +933,16 @@ struct pgbt_tree {
 
 namespace {
 
+// Nodes that every construction array holds: the buffers round their own sizes up, so the arrays of
+// three and eight entries a node may hold fewer nodes than the others.
+size_t node_capacity(const pgbt_tree* T) {
+    return std::min({T->bfirst.n, T->bcount.n, T->bparent.n, T->bhalf.n, T->bchild.n / 8, T->bc.n / 3});
+}
+
 bool grow_nodes(pgbt_tree* T, size_t need, size_t keep) {
-    if (need <= T->bfirst.n) return true;
-    const size_t want = std::max(need, 2 * T->bfirst.n);
+    const size_t cap = node_capacity(T);
+    if (need <= cap) return true;
+    const size_t want = std::max(need, 2 * cap);
     PGB_CUDA_OR(g_err, LIB, T->bfirst.grow_keep(want, keep, T->s), return false);
     PGB_CUDA_OR(g_err, LIB, T->bcount.grow_keep(want, keep, T->s), return false);
     PGB_CUDA_OR(g_err, LIB, T->bparent.grow_keep(want, keep, T->s), return false);
