@@ -173,9 +173,10 @@ struct Group {
 };
 
 // Number of j-chunks for one item of `itiles` equal i-tiles on `slots` resident CTAs: the
-// persistent CTAs run ceil(itiles*nch/slots) waves of tasks of nj/nch pairs per i, so the time
-// is proportional to waves/nch; a small penalty per chunk accounts for the partial-row
-// reduction.  Chunks hold at least `minj` j and there are at most `maxch` of them.
+// persistent CTAs run ceil(itiles*nch/slots) waves of tasks of nj/nch pairs per i, each of which
+// costs about 256 j more than its pairs (its start, lane sums and partial row; 2086 i x 2134 j on the
+// 512-thread Hermite CTAs: 13 chunks, three waves, 24.9 us, 4 chunks, one wave, 17.4).  Chunks hold at
+// least `minj` j and there are at most `maxch` of them.
 inline int best_nch(long long itiles, long long nj, long long slots, int maxch, int minj = 128) {
     long long hi = nj / minj;
     if (hi > maxch) hi = maxch;
@@ -184,7 +185,7 @@ inline int best_nch(long long itiles, long long nj, long long slots, int maxch, 
     int arg = 1;
     for (long long n = 1; n <= hi; n++) {
         long long waves = (itiles * n + slots - 1) / slots;
-        double cost = (double)waves / (double)n * (1.0 + 0.002 * (double)n);
+        double cost = (double)waves * ((double)nj / (double)n + 256.0);
         if (cost < best) {
             best = cost;
             arg = (int)n;
@@ -193,29 +194,57 @@ inline int best_nch(long long itiles, long long nj, long long slots, int maxch, 
     return arg;
 }
 
+// The same for the j-paired kernels, whose chunks are whole j-tiles of `tile` records: a partial
+// tile runs their loop with a run-time count and leaves j-lanes idle.  They are bound by the SM's FMA
+// pipe from two resident CTAs on, so the time is that of the SM with the most tasks, ceil(tasks /
+// sms) chunks, whatever the number of resident CTAs; a task costs about 150 j more than its chunk, a
+// chunk to reduce about 2, and the last tasks of an SM, which run with fewer beside them, `tail` of a
+// chunk (0.2).  Measured for 2048 x 65536 (16 i-tiles): 27 chunks 187.2 us (the wave model), 37: 184.8,
+// 64 (1024 j): 178.8, 128: 189.0; 4096 x 16384 (32 i-tiles): 9: 101.3, 12 and 16: 111.6 (3 and 4
+// tasks on an SM), 18: 103.0; 3000 x 16384: 12: 80.5, 43: 93.7; 4096 x 65536: 9: 356, 32: 334.
+// Returns the chunk's length, a multiple of tile (or nj).
+inline long long best_tile_chunk(long long itiles, long long nj, long long sms, int tile, int maxch, double tail) {
+    const long long ntile = (nj + tile - 1) / tile;
+    if (ntile <= 1) return nj > 0 ? nj : 1;
+    double best = 1e300;
+    long long arg = ntile;
+    for (long long c = 1; c <= ntile; c++) {
+        const long long n = (ntile + c - 1) / c;
+        if (n > maxch) continue;
+        const long long tasks = itiles * n, k = (tasks + sms - 1) / sms;
+        const double cost = (double)k * (double)(c * tile + 150) + tail * (double)(c * tile) + 2.0 * (double)n;
+        if (cost < best) {
+            best = cost;
+            arg = c;
+        }
+    }
+    return arg * tile;
+}
+
 // Split [0,ni) x [0,nj) into tasks of at most `itile` i and about `jchunk` j, appending to
-// `tasks`/`groups`.  Offsets are added to i0/j0.  Returns the partial rows used.
+// `tasks`/`groups`.  Offsets are added to i0/j0.  The chunks are near-equal numbers of whole
+// `align`-record tiles (the last one takes what is left).  Returns the partial rows used.
 inline int plan_item(std::vector<Task>& tasks, std::vector<Group>& groups, int i_off, int ni,
-                     int j_off, int nj, int itile, int jchunk, int slot_base, int aux = 0) {
+                     int j_off, int nj, int itile, int jchunk, int slot_base, int align = 1) {
     if (ni <= 0) return 0;
-    int nch = (nj + jchunk - 1) / jchunk;
+    const int units = (int)(((long long)nj + align - 1) / align);
+    int nch = (int)(((long long)nj + jchunk - 1) / jchunk);
+    if (nch > units) nch = units;
     if (nch < 1) nch = 1;
     int used = 0;
     for (int it = 0; it < ni; it += itile) {
         int nii = ni - it < itile ? ni - it : itile;
         if (nch == 1) {
-            tasks.push_back(Task{i_off + it, nii, j_off, nj, -1, 0, -1, aux});
+            tasks.push_back(Task{i_off + it, nii, j_off, nj, -1, 0, -1, 0});
             continue;
         }
         int g = (int)groups.size();
         groups.push_back(Group{i_off + it, nii, nch, slot_base + used});
-        // near-equal chunks, each a multiple of 32 j where possible
-        long long base = (long long)nj / nch;
-        int rem = nj - (int)(base * nch);
+        const int base = units / nch, rem = units - base * nch;
         int j = 0;
         for (int c = 0; c < nch; c++) {
-            int len = (int)base + (c < rem ? 1 : 0);
-            tasks.push_back(Task{i_off + it, nii, j_off + j, len, g, c, slot_base + used + c, aux});
+            const int len = std::min(nj - j, (base + (c < rem ? 1 : 0)) * align);
+            tasks.push_back(Task{i_off + it, nii, j_off + j, len, g, c, slot_base + used + c, 0});
             j += len;
         }
         used += nch;

@@ -83,104 +83,117 @@ bool ensure_device() {
 }
 
 // ------------------------------------------------------------------------------------------
-// kernel configurations: (threads per CTA, i per thread, j-lanes); i-tile = NT/JL*IPT
+// kernel configurations (cfg_kernel: threads per CTA, i per thread, j-lanes, form).  CFG_MED, CFG_128x1
+// and CFG_*J have a j-paired form (1: g6_jpair, 2: stage-ordered g6_jquad2, 3: g6_jpair with the best
+// j-quad kept) for double-float positions without neighbour lists.
 
 enum Cfg {
     CFG_SMALL = 0, CFG_MED = 1, CFG_LARGE = 2, CFG_128x1 = 3, CFG_128x4 = 4, CFG_256x2 = 5,
     CFG_128x2J = 6, CFG_256x2J = 7, CFG_128x4J = 8, CFG_128x2JS = 9, NCFG = 10
 };
-constexpr int CFG_NT[NCFG] = {512, 256, 128, 128, 128, 256, 128, 256, 128, 128};
-constexpr int CFG_IPT[NCFG] = {1, 1, 2, 1, 4, 2, 2, 2, 4, 2};
-constexpr int CFG_JL[NCFG] = {8, 2, 1, 1, 1, 1, 1, 1, 1, 1};
-// j-paired form (1: g6_jpair, 2: stage-ordered g6_jquad2): used with double-float positions and
-// without neighbour lists; the other variants of these configurations run the i-paired form
-constexpr int CFG_JP[NCFG] = {0, 0, 0, 0, 0, 0, 1, 1, 1, 2};
-inline int cfg_itile(int c) { return CFG_NT[c] / CFG_JL[c] * CFG_IPT[c]; }
 constexpr int ITILE_MAX = 512;
 
-template <int NT, int IPT, int JL, bool FF, int JP = 0>
-int occ_of(bool nn, bool nbl) {
-    static int v[4] = {0, 0, 0, 0};
-    int k = (nn ? 1 : 0) + (nbl ? 2 : 0);
-    if (!v[k]) {
+// One kernel of a configuration: a launch (info == nullptr), or what the host needs to know of it: its
+// resident CTAs per SM, j records and i a tile, and forms.
+struct KernelInfo {
+    int occ = 0, tile = 0, itile = 0;
+    bool paired = false;    // the j-paired form
+    double tail = 0.2;      // best_tile_chunk's (the stage-ordered form loses more with few CTAs on an SM:
+                            // 65536 x 65536 in 8 chunks 4996 us, in 16 to 19 4664)
+    bool resolve = false;   // leaves the nearest-neighbour lookups of split i-tiles to g6_resolve_kernel
+};
+template <int NT, int IPT, int JL, bool FF, bool NN, bool NBL, int JP>
+void one_kernel(int grid, const G6Args& a, cudaStream_t s, KernelInfo* info) {
+    auto k = g6_kernel<NT, IPT, JL, FF, NN, NBL, JP>;
+    if (info) {
         int b = 0;
-        if (k == 0)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, g6_kernel<NT, IPT, JL, FF, false, false, JP>, NT, 0);
-        if (k == 1)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, g6_kernel<NT, IPT, JL, FF, true, false, JP>, NT, 0);
-        if (k == 2)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, g6_kernel<NT, IPT, JL, FF, false, true, JP>, NT, 0);
-        if (k == 3)
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, g6_kernel<NT, IPT, JL, FF, true, true, JP>, NT, 0);
-        v[k] = b > 0 ? b : 1;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k, NT, 0);
+        info->occ = b > 0 ? b : 1;
+        info->tile = g6_tile_j<NT, JL, g6_uses_jp<IPT, FF, NBL, JP>()>();
+        info->itile = NT / JL * IPT;
+        info->paired = g6_uses_jp<IPT, FF, NBL, JP>();
+        info->tail = JP == 2 ? 0.5 : 0.2;
+        info->resolve = NN && !NBL && IPT % 2 == 0 && !g6_quad_min<IPT, FF, NBL, JP>();
+        return;
     }
-    return v[k];
+    k<<<grid, NT, 0, s>>>(a);
 }
 
-template <bool FF>
-int occupancy_ff(int cfg, bool nn, bool nbl) {
+// CFG_MED: the j-paired form over two j-lanes (two i per thread) where it applies, else one i per
+// thread over two lanes; the i-tile is the same.
+template <bool FF, bool NN, bool NBL>
+void med_kernel(int grid, const G6Args& a, cudaStream_t s, KernelInfo* info) {
+    if constexpr (FF && !NBL) one_kernel<128, 2, 2, FF, NN, NBL, 3>(grid, a, s, info);
+    else one_kernel<256, 1, 2, FF, NN, NBL, 0>(grid, a, s, info);
+}
+
+// CFG_128x1: the j-paired form of CFG_128x2J with the best j-quad kept (256 i a tile, no lookup
+// kernel) where it applies, else one i per thread.
+template <bool FF, bool NN, bool NBL>
+void quad_kernel(int grid, const G6Args& a, cudaStream_t s, KernelInfo* info) {
+    if constexpr (FF && !NBL) one_kernel<128, 2, 1, FF, NN, NBL, 3>(grid, a, s, info);
+    else one_kernel<128, 1, 1, FF, NN, NBL, 0>(grid, a, s, info);
+}
+
+template <bool FF, bool NN, bool NBL>
+void cfg_kernel(int cfg, int grid, const G6Args& a, cudaStream_t s, KernelInfo* info) {
     switch (cfg) {
-        case CFG_SMALL: return occ_of<512, 1, 8, FF>(nn, nbl);
-        case CFG_MED: return occ_of<256, 1, 2, FF>(nn, nbl);
-        case CFG_128x1: return occ_of<128, 1, 1, FF>(nn, nbl);
-        case CFG_128x4: return occ_of<128, 4, 1, FF>(nn, nbl);
-        case CFG_256x2: return occ_of<256, 2, 1, FF>(nn, nbl);
-        case CFG_128x2J: return occ_of<128, 2, 1, FF, 1>(nn, nbl);
-        case CFG_256x2J: return occ_of<256, 2, 1, FF, 1>(nn, nbl);
-        case CFG_128x4J: return occ_of<128, 4, 1, FF, 1>(nn, nbl);
-        case CFG_128x2JS: return occ_of<128, 2, 1, FF, 2>(nn, nbl);
-        default: return occ_of<128, 2, 1, FF>(nn, nbl);
+        case CFG_SMALL: one_kernel<512, 1, 8, FF, NN, NBL, 0>(grid, a, s, info); break;
+        case CFG_MED: med_kernel<FF, NN, NBL>(grid, a, s, info); break;
+        case CFG_128x1: quad_kernel<FF, NN, NBL>(grid, a, s, info); break;
+        case CFG_128x4: one_kernel<128, 4, 1, FF, NN, NBL, 0>(grid, a, s, info); break;
+        case CFG_256x2: one_kernel<256, 2, 1, FF, NN, NBL, 0>(grid, a, s, info); break;
+        case CFG_128x2J: one_kernel<128, 2, 1, FF, NN, NBL, 1>(grid, a, s, info); break;
+        case CFG_256x2J: one_kernel<256, 2, 1, FF, NN, NBL, 1>(grid, a, s, info); break;
+        case CFG_128x4J: one_kernel<128, 4, 1, FF, NN, NBL, 1>(grid, a, s, info); break;
+        case CFG_128x2JS: one_kernel<128, 2, 1, FF, NN, NBL, 2>(grid, a, s, info); break;
+        default: one_kernel<128, 2, 1, FF, NN, NBL, 0>(grid, a, s, info); break;
     }
 }
 
-int occupancy(int cfg, bool ff, bool nn, bool nbl) {
-    return ff ? occupancy_ff<true>(cfg, nn, nbl) : occupancy_ff<false>(cfg, nn, nbl);
-}
-
-template <int NT, int IPT, int JL, bool FF, int JP = 0>
-void launch_cfg(bool nn, bool nbl, int grid, const G6Args& a, cudaStream_t s) {
-    if (nn && nbl) g6_kernel<NT, IPT, JL, FF, true, true, JP><<<grid, NT, 0, s>>>(a);
-    else if (nn) g6_kernel<NT, IPT, JL, FF, true, false, JP><<<grid, NT, 0, s>>>(a);
-    else if (nbl) g6_kernel<NT, IPT, JL, FF, false, true, JP><<<grid, NT, 0, s>>>(a);
-    else g6_kernel<NT, IPT, JL, FF, false, false, JP><<<grid, NT, 0, s>>>(a);
-}
-
-template <bool FF>
-void launch_ff(int cfg, bool nn, bool nbl, int grid, const G6Args& a, cudaStream_t s) {
-    switch (cfg) {
-        case CFG_SMALL: launch_cfg<512, 1, 8, FF>(nn, nbl, grid, a, s); break;
-        case CFG_MED: launch_cfg<256, 1, 2, FF>(nn, nbl, grid, a, s); break;
-        case CFG_128x1: launch_cfg<128, 1, 1, FF>(nn, nbl, grid, a, s); break;
-        case CFG_128x4: launch_cfg<128, 4, 1, FF>(nn, nbl, grid, a, s); break;
-        case CFG_256x2: launch_cfg<256, 2, 1, FF>(nn, nbl, grid, a, s); break;
-        case CFG_128x2J: launch_cfg<128, 2, 1, FF, 1>(nn, nbl, grid, a, s); break;
-        case CFG_256x2J: launch_cfg<256, 2, 1, FF, 1>(nn, nbl, grid, a, s); break;
-        case CFG_128x4J: launch_cfg<128, 4, 1, FF, 1>(nn, nbl, grid, a, s); break;
-        case CFG_128x2JS: launch_cfg<128, 2, 1, FF, 2>(nn, nbl, grid, a, s); break;
-        default: launch_cfg<128, 2, 1, FF>(nn, nbl, grid, a, s); break;
+void any_kernel(int cfg, bool ff, bool nn, bool nbl, int grid, const G6Args& a, cudaStream_t s, KernelInfo* info) {
+    switch ((ff ? 4 : 0) | (nn ? 2 : 0) | (nbl ? 1 : 0)) {
+        case 0: cfg_kernel<false, false, false>(cfg, grid, a, s, info); break;
+        case 1: cfg_kernel<false, false, true>(cfg, grid, a, s, info); break;
+        case 2: cfg_kernel<false, true, false>(cfg, grid, a, s, info); break;
+        case 3: cfg_kernel<false, true, true>(cfg, grid, a, s, info); break;
+        case 4: cfg_kernel<true, false, false>(cfg, grid, a, s, info); break;
+        case 5: cfg_kernel<true, false, true>(cfg, grid, a, s, info); break;
+        case 6: cfg_kernel<true, true, false>(cfg, grid, a, s, info); break;
+        default: cfg_kernel<true, true, true>(cfg, grid, a, s, info); break;
     }
 }
+
+KernelInfo kernel_info(int cfg, bool ff, bool nn, bool nbl) {
+    static std::mutex mu;
+    static KernelInfo cache[NCFG][8];
+    std::lock_guard<std::mutex> g(mu);
+    KernelInfo& v = cache[cfg][(ff ? 4 : 0) | (nn ? 2 : 0) | (nbl ? 1 : 0)];
+    if (!v.occ) any_kernel(cfg, ff, nn, nbl, 0, G6Args{}, nullptr, &v);
+    return v;
+}
+int occupancy(int cfg, bool ff, bool nn, bool nbl) { return kernel_info(cfg, ff, nn, nbl).occ; }
 
 cudaError_t launch_kernel(int cfg, bool ff, bool nn, bool nbl, int grid, const G6Args& a, cudaStream_t s) {
-    if (ff) launch_ff<true>(cfg, nn, nbl, grid, a, s);
-    else launch_ff<false>(cfg, nn, nbl, grid, a, s);
+    any_kernel(cfg, ff, nn, nbl, grid, a, s, nullptr);
     return cudaGetLastError();
 }
 
-// Whether a force launch of this shape leaves nearest-neighbour lookups to g6_resolve_kernel:
-// the tile-minimum search (two or four i per thread; one j-lane), split i-tiles (ngroups > 0),
-// j addresses below the G6_NN_TILE mark (g6_task's `defer`).
-bool needs_resolve(int cfg, bool nn, bool nbl, int ngroups, int jn) {
-    return nn && !nbl && ngroups > 0 && CFG_IPT[cfg] % 2 == 0 && CFG_JL[cfg] == 1 && jn < G6_NN_TILE;
+// Whether a force launch of this shape leaves nearest-neighbour lookups to g6_resolve_kernel (the
+// kernel's tile-minimum search, split i-tiles (ngroups > 0), j addresses below the G6_NN_TILE
+// mark: g6_task's `defer`).
+bool needs_resolve(int cfg, bool ff, bool nn, bool nbl, int ngroups, int jn) {
+    return nn && ngroups > 0 && jn < G6_NN_TILE && kernel_info(cfg, ff, nn, nbl).resolve;
 }
 
 // The deferred nearest-neighbour lookups of a force launch (after it, on the same stream).
 cudaError_t launch_resolve(int cfg, bool ff, bool nn, bool nbl, int ngroups, const G6Args& a, cudaStream_t s) {
-    if (!needs_resolve(cfg, nn, nbl, ngroups, a.jn)) return cudaSuccess;
+    if (!needs_resolve(cfg, ff, nn, nbl, ngroups, a.jn)) return cudaSuccess;
     constexpr int rpb = 128 / G6_RES_LANES;
     const long long grid = (long long)ngroups * ((a.itile + rpb - 1) / rpb);
-    if (ff) g6_resolve_kernel<true><<<(unsigned)grid, 128, 0, s>>>(a, ngroups, CFG_NT[cfg]);
-    else g6_resolve_kernel<false><<<(unsigned)grid, 128, 0, s>>>(a, ngroups, CFG_NT[cfg]);
+    const int tile = kernel_info(cfg, ff, nn, nbl).tile;
+    if (ff) g6_resolve_kernel<true><<<(unsigned)grid, 128, 0, s>>>(a, ngroups, tile);
+    else g6_resolve_kernel<false><<<(unsigned)grid, 128, 0, s>>>(a, ngroups, tile);
     return cudaGetLastError();
 }
 
@@ -282,13 +295,56 @@ bool dx_ff() {
     return v == 1;
 }
 
-// Forced configuration for tuning sweeps (PGB_G6_CFG = 0..3), else by i count.
-int pick_cfg(long long ni_max) {
+// The default configuration (PGB_G6_CFG forces one for sweeps) of a call or plan of one item of ni i
+// against nj j.  With double-float positions and no neighbour lists: SMALL (512 threads, 8 j-lanes)
+// while the launch's latency counts more than its pairs, MED (j-paired, 128 i a tile, two j-lanes)
+// for the middle, the stage-ordered j-paired form for the largest.  Measured (us, SMALL / MED / JS, and
+// the scalar two-i form that was the default from 4097 i up):
+//   777 x 4096     14.6 /   22.8 /   41    777 x 65536    98.6 /  102   /  127
+//   2086 x 2134    17.4 /   23.1 /   -     3000 x 4096    29.3 /   33.4 /   51
+//   1500 x 16384   49.9 /   51.5 /   70    2086 x 16384   70.2 /   64.4 /   82
+//   4096 x 16384  140   /  101   /  121    8192 x 16384  244   /  177   /  198   (220)
+//   8192 x 65536  876   /  646   /  632 (749)   16384 x 16384  458 / 329 / 344 (399)
+//   16384 x 65536  1718 / 1260 / 1208 (1457)    65536 x 65536  6754 / 4890 / 4664 (5488)
+int pick_cfg(long long ni, long long nj, bool ff, bool nbl) {
     static int forced = env_int("PGB_G6_CFG", -1, -1, NCFG - 1);
     if (forced >= 0) return forced;
-    if (ni_max <= 64) return CFG_SMALL;
-    if (ni_max <= 4096) return CFG_MED;
+    if (ff && !nbl) {
+        if (ni <= 3072 && ni * nj <= (ni <= 1024 ? 48LL << 20 : 24LL << 20)) return CFG_SMALL;
+        return ni * nj < (1LL << 29) ? CFG_MED : CFG_128x2JS;
+    }
+    if (ni <= 64) return CFG_SMALL;
+    if (ni <= 4096) return CFG_MED;
     return CFG_LARGE;
+}
+
+// The same for a batch of several items, by the i count that the average pair sees: MED's smaller
+// i-tiles up to 6000, then CFG_128x1's j-paired form (us, MED / 128x1 / the scalar form that was the
+// default: 40 clusters of 300 to 5000 particles 220 / 234 / 327, 96 of 64 to 2048 110 / 122 / 192, 96 of
+// 256 to 16384 4352 / 4227 / 5136).
+int pick_batch_cfg(int nitem, const int* items, bool ff) {
+    double w = 0.0, wi = 0.0;
+    long long nimax = 0, njmax = 0, total_i = 0;
+    for (int k = 0; k < nitem; k++) {
+        const long long ni = items[4 * k + 1], nj = items[4 * k + 3];
+        nimax = std::max(nimax, ni);
+        njmax = std::max(njmax, nj);
+        total_i += ni;
+        w += (double)ni * (double)nj;
+        wi += (double)ni * (double)nj * (double)ni;
+    }
+    if (nitem == 1) return pick_cfg(nimax, njmax, ff, false);
+    if (!ff) return pick_cfg(std::max(nimax, total_i / 4), njmax, ff, false);
+    static int forced = env_int("PGB_G6_CFG", -1, -1, NCFG - 1);
+    if (forced >= 0) return forced;
+    return wi <= 6000.0 * w ? CFG_MED : CFG_128x1;
+}
+
+// The chunk length of a single item: the j-paired kernels' whole tiles, else the wave model's.
+long long model_chunk(const KernelInfo& K, long long itiles, int nj, int slots, int maxch) {
+    if (K.paired) return best_tile_chunk(itiles, nj, sm_count(g_device), K.tile, maxch, K.tail);
+    const int nch = best_nch(itiles, nj, slots, maxch);
+    return (nj + nch - 1) / nch;
 }
 
 // Plan one batch of items ([k][4] = i_off, i_cnt, j_off, j_cnt) for a configuration:
@@ -296,8 +352,9 @@ int pick_cfg(long long ni_max) {
 // (their partial rows are summed by the cooperative reduction of the group's last CTA).
 long long plan_items(std::vector<Task>& tasks, std::vector<Group>& groups, int& rows, int nitem, const int* items,
                      int cfg, bool ff, bool nn, bool nbl, int nch_fixed = 0) {
-    int slots = sm_count(g_device) * occupancy(cfg, ff, nn, nbl);
-    int itile = cfg_itile(cfg);
+    const KernelInfo K = kernel_info(cfg, ff, nn, nbl);
+    int slots = sm_count(g_device) * K.occ;
+    int itile = K.itile;
     long long work = 0;
     for (int k = 0; k < nitem; k++) {
         long long ni = items[4 * k + 1];
@@ -319,15 +376,17 @@ long long plan_items(std::vector<Task>& tasks, std::vector<Group>& groups, int& 
             // the autotuner's (nch_fixed)
             long long itiles = (ni + itile - 1) / itile;
             static const int forced_nch = env_int("PGB_G6_NCH", 0, 0, 4096);   // profiling: a pinned count
-            int nch = forced_nch > 0 ? forced_nch : nch_fixed > 0 ? nch_fixed : best_nch(itiles, nj, slots, (int)maxch);
-            jc = (nj + nch - 1) / nch;
+            const int nch = forced_nch > 0 ? forced_nch : nch_fixed;
+            if (nch > 0) jc = (nj + nch - 1) / nch;
+            else jc = model_chunk(K, itiles, nj, slots, (int)maxch);
         } else {
             jc = per_task / itile;
             if (jc < 128) jc = 128;
             if (jc * maxch < nj) jc = (nj + maxch - 1) / maxch;
         }
         if (jc > nj) jc = nj > 0 ? nj : 1;
-        rows += plan_item(tasks, groups, items[4 * k], ni, items[4 * k + 2], nj, itile, (int)jc, rows);
+        rows += plan_item(tasks, groups, items[4 * k], ni, items[4 * k + 2], nj, itile, (int)jc, rows,
+                          K.paired ? K.tile : 1);
         inter += (long long)ni * nj;
     }
     std::stable_sort(tasks.begin(), tasks.end(), [](const Task& a, const Task& b) {
@@ -589,9 +648,9 @@ bool run_force(int nj, int ni, float eps2, bool nn, bool nbl) {
     }
     G6Out* out_dev = S.outh_dev;
     if (ni <= G6_SMALL_MAXI && nj > 0) return run_small(nj, ni, eps2, nn, nbl, out_dev);
-    const int cfg = pick_cfg(ni);
     const bool ff = dx_ff();
-    const int itile = cfg_itile(cfg);
+    const int cfg = pick_cfg(ni, nj, ff, nbl);
+    const int itile = kernel_info(cfg, ff, nn, nbl).itile;
     const int slots = sm_count(g_device) * occupancy(cfg, ff, nn, nbl);
     static const int maxch = env_int("PGB_G6_MAXCHUNKS", 512, 1, 4096);
     const int itiles = (ni + itile - 1) / itile;
@@ -1057,16 +1116,11 @@ PGB_EXPORT int pgb6_plan_create(pgb6_plan** out, int nitem, const int* items, in
     auto* P = new pgb6_plan();
     P->nn = (flags & PGB6_NN) != 0;
     P->ff = (flags & PGB6_POS_F64) == 0;
-    long long nimax = 0;
-    for (int k = 0; k < nitem; k++) nimax = std::max<long long>(nimax, items[4 * k + 1]);
-    // many small items fill the GPU with short tiles; large ones prefer 2 i per thread
-    long long total_i = 0;
-    for (int k = 0; k < nitem; k++) total_i += items[4 * k + 1];
     P->items.assign(items, items + 4 * (size_t)nitem);
     P->jend = items_jend(nitem, items);
     P->shape_key = shape_key(nitem, items, P->ff, P->nn);
     const Tuned tuned = tuned_cfg(P->shape_key);
-    P->cfg = tuned.cfg >= 0 ? tuned.cfg : pick_cfg(nitem > 1 ? std::max<long long>(nimax, total_i / 4) : nimax);
+    P->cfg = tuned.cfg >= 0 ? tuned.cfg : pick_batch_cfg(nitem, items, P->ff);
     P->nch = tuned.cfg >= 0 ? tuned.nch : 0;
     P->interactions = plan_items(P->tasks, P->groups, P->rows, nitem, items, P->cfg, P->ff, P->nn, false, P->nch);
     cudaStream_t s = nullptr;
@@ -1096,7 +1150,7 @@ PGB_EXPORT int pgb6_plan_chunks(const pgb6_plan* P) {
 // split i-tiles when the plan's configuration defers them.
 PGB_EXPORT int pgb6_plan_kernels(const pgb6_plan* P) {
     if (!P || P->tasks.empty()) return 0;
-    return 1 + (needs_resolve(P->cfg, P->nn, false, (int)P->groups.size(), P->jend) ? 1 : 0);
+    return 1 + (needs_resolve(P->cfg, P->ff, P->nn, false, (int)P->groups.size(), P->jend) ? 1 : 0);
 }
 
 // Device-resident launch (capturable in a CUDA graph): ipart = G6I[], jpred = G6PredJ[],
@@ -1122,7 +1176,7 @@ PGB_EXPORT int pgb6_plan_launch(pgb6_plan* P, const void* ipart, const void* jpr
     a.group_counters = P->st.dgcnt.p;
     a.partial = P->st.dpart.p;
     a.out = (G6Out*)out;
-    a.itile = cfg_itile(P->cfg);
+    a.itile = kernel_info(P->cfg, P->ff, P->nn, false).itile;
     a.bundle_counters = P->st.bundle_counters();
     a.nb_count = nullptr;
     a.nb_list = nullptr;
@@ -1267,9 +1321,9 @@ PGB_EXPORT int pgb6_plan_tune(pgb6_plan* P, const void* ipart, const void* jpred
         const int ni = P->items[1], nj = P->items[3];
         for (size_t r = 0; r < by_cfg.size() && r < 3; r++) {
             const int cfg = by_cfg[r].second;
-            const int itile = cfg_itile(cfg);
-            const int slots = sm_count(g_device) * occupancy(cfg, P->ff, P->nn, false);
-            const int m = best_nch((ni + itile - 1) / itile, nj, slots, maxch);
+            const KernelInfo K = kernel_info(cfg, P->ff, P->nn, false);
+            const long long jc = model_chunk(K, (ni + K.itile - 1) / K.itile, nj, sm_count(g_device) * K.occ, maxch);
+            const int m = (int)((nj + jc - 1) / jc);
             for (int nch : chunk_candidates(m, nj, maxch)) {
                 if (nch == m) continue;   // timed above
                 float t;
@@ -1470,8 +1524,12 @@ PGB_EXPORT int pgb6_force_noalloc(const void* ipart, int ni, const void* jpred, 
     if (ni == 0) return PGB_OK;
     if (!ensure_device()) return PGB_ERR_NOGPU;
     const bool nn = (flags & PGB6_NN) != 0, ff = (flags & PGB6_POS_F64) == 0;
-    const int cfg = pick_cfg(ni);
-    const int itile = cfg_itile(cfg);
+    int cfg = pick_cfg(ni, nj, ff, false);
+    int itile = kernel_info(cfg, ff, nn, false).itile;
+    if (ni > (long long)NOALLOC_MAX_ITILES * itile) {   // too many small tiles: the 256-particle tile
+        cfg = ff ? CFG_128x2JS : CFG_LARGE;
+        itile = kernel_info(cfg, ff, nn, false).itile;
+    }
     const long long itiles = (ni + (long long)itile - 1) / itile;
     if (itiles > NOALLOC_MAX_ITILES) {
         raise(g_err, LIB, PGB_ERR_CAPACITY, "pgb6_force_noalloc: ni = %d exceeds the fixed scratch (%d i-tiles of %d)",

@@ -530,6 +530,22 @@ __device__ __forceinline__ int g6_rescan(const G6PredJ* __restrict__ jpred, int 
     return -1;
 }
 
+// The address of the nearest neighbour whose j-quad the j-paired form recorded (b: the quad's first
+// record; -1: no candidate): the first of the quad's records with that key.
+template <bool FF>
+__device__ __forceinline__ int g6_quad_lookup(const G6Args& A, int i, float key, int b) {
+    if (b < 0) return -1;
+    const G6I P = A.ipart[i];
+    G6PredJ J[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) J[u] = A.jpred[min(b + u, A.jn - 1)];
+    int found = -1;
+#pragma unroll
+    for (int u = 3; u >= 0; u--)
+        if (g6_key<FF>(J[u], P.p, P.id, A.eps2) == key) found = b + u;
+    return found;
+}
+
 __device__ __forceinline__ G6Out g6_finish(const G6Out& s) {
     G6Out o;
     o.ax = S_ACC * s.ax;
@@ -671,11 +687,21 @@ struct BoolC {
 // Shared memory of a g6_kernel CTA: the j-tile (as records, or as field arrays in the j-paired
 // form, which also keeps its threads' FP64 sums there: 7 per i) and, after the tile loop, NT
 // G6Out for the lane and group reductions.
-template <int NT, int IPT, bool JP>
+template <int NT, int IPT, bool JP, int NJ>
 constexpr int g6_smem_bytes() {
-    return JP ? (int)((sizeof(G6TileSoA<NT>) + 15) / 16 * 16 + 7 * IPT * NT * sizeof(double))
+    return JP ? (int)((sizeof(G6TileSoA<NJ>) + 15) / 16 * 16 + 7 * IPT * NT * sizeof(double))
               : NT * (int)sizeof(G6Out);
 }
+
+// Whether a kernel variant runs the j-paired form, and its j records a tile: one a thread, or 64 a
+// lane where the j-paired form splits the tile over lanes.
+template <int IPT, bool FF, bool NBL, int JP>
+constexpr bool g6_uses_jp() { return JP != 0 && FF && !NBL && (IPT == 2 || IPT == 4); }
+// JP 3 is the j-pair order of JP 1 with the best j-quad kept instead of the best tile (see g6_task).
+template <int IPT, bool FF, bool NBL, int JP>
+constexpr bool g6_quad_min() { return JP == 3 && g6_uses_jp<IPT, FF, NBL, JP>(); }
+template <int NT, int JL, bool USE_JP>
+constexpr int g6_tile_j() { return USE_JP && JL > 1 ? 64 * JL : NT; }
 
 // Thread layout of a CTA: NT threads = JL j-lanes x ISL i-slots (ISL = NT/JL, whole warps per
 // lane so that the shared-memory j reads stay warp-broadcasts).  A thread owns IPT i-particles
@@ -690,21 +716,28 @@ constexpr int g6_smem_bytes() {
 // (a j id inside the i-tile's id range, one __syncthreads_or at the staging barrier); only such
 // tiles run the self-pair mask.  With two i per thread (IPT even) the nearest neighbour is
 // found as a tile minimum (see g6_pair) and its address recovered once per i and task by
-// g6_rescan.  JP selects the j-paired form (1: g6_jpair, 2: g6_jquad2 for two i per thread;
-// double-float positions, no neighbour lists, one j-lane); otherwise the j-tile is an array of
-// G6PredJ records.
+// g6_rescan.  JP selects the j-paired form (1, 3: g6_jpair, 2: g6_jquad2 for two i per thread;
+// double-float positions, no neighbour lists; with j-lanes, lane l takes the tile's j-quads l,
+// l + JL, ...); otherwise the j-tile is an array of G6PredJ records.  JP 3 keeps the best j-quad
+// (a compare and two selects per quad on the ALU pipe, which the FMA-bound loop has free) instead
+// of the best tile: the address is then one look at four records, by the task that owns its i or
+// by the CTA that completes the group, and no g6_resolve_kernel follows.  With the lookups: 96
+// clusters of 256 to 16384 particles 4475 -> 4227 us, 777 x 4096 43 -> 37, 65536 x 65536 4795 -> 4791;
+// the stage-ordered loop (JP 2) would lose 2.6 % to it on the largest call (4686 -> 4810 us).
 template <int NT, int IPT, int JL, bool FF, bool NN, bool NBL, int JP = 0>
 __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned char* smem) {
-    static_assert(JL == 1 || IPT == 1, "j-lanes are used with one i per thread");
     constexpr int ISL = NT / JL;
     constexpr bool PAIRED = (IPT % 2 == 0);
-    constexpr bool USE_JP = JP && FF && !NBL && (IPT == 2 || IPT == 4) && JL == 1;
-    constexpr bool TILEMIN = NN && !NBL && PAIRED;
+    constexpr bool USE_JP = g6_uses_jp<IPT, FF, NBL, JP>();
+    constexpr int NJ = g6_tile_j<NT, JL, USE_JP>();
+    static_assert(JL == 1 || IPT == 1 || USE_JP, "j-lanes are used with one i per thread or the j-paired form");
+    constexpr bool QUADMIN = g6_quad_min<IPT, FF, NBL, JP>() && NN;
+    constexpr bool TILEMIN = NN && !NBL && PAIRED && !QUADMIN;
     G6PredJ* sj = reinterpret_cast<G6PredJ*>(smem);
-    G6TileSoA<NT>* sa = reinterpret_cast<G6TileSoA<NT>*>(smem);
+    G6TileSoA<NJ>* sa = reinterpret_cast<G6TileSoA<NJ>*>(smem);
     // j-paired form: the FP64 sums of thread t, i k, component c at Ssh[(k * 7 + c) * NT + t]
     // (updated once per G6_FOLD j; kept out of the registers)
-    double* Ssh = reinterpret_cast<double*>(smem + (sizeof(G6TileSoA<NT>) + 15) / 16 * 16);
+    double* Ssh = reinterpret_cast<double*>(smem + (sizeof(G6TileSoA<NJ>) + 15) / 16 * 16);
     G6Out* red = reinterpret_cast<G6Out*>(smem);
     __shared__ int s_idr[2];
     const int slot = threadIdx.x % ISL;
@@ -774,8 +807,8 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
         }
     }
 
-    for (int jt = 0; jt < T.nj; jt += NT) {
-        const int nt = min(NT, T.nj - jt);
+    for (int jt = 0; jt < T.nj; jt += NJ) {
+        const int nt = min(NJ, T.nj - jt);
         __syncthreads();
         const int idlo = s_idr[0], idhi = s_idr[1];
         bool mine = false;
@@ -784,21 +817,23 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
             // fields of the tile's records, padded to a multiple of 4 with massless copies of
             // the tile's first record (they add exact zeros, and their key repeats that record's)
             nt4 = (nt + 3) & ~3;
-            if (threadIdx.x < nt4) {
-                const bool real = threadIdx.x < nt;
-                const G6PredJ r = A.jpred[T.j0 + jt + (real ? threadIdx.x : 0)];
-                sa->xh[threadIdx.x] = r.p.f.xh;
-                sa->yh[threadIdx.x] = r.p.f.yh;
-                sa->zh[threadIdx.x] = r.p.f.zh;
-                sa->xl[threadIdx.x] = r.p.f.xl;
-                sa->yl[threadIdx.x] = r.p.f.yl;
-                sa->zl[threadIdx.x] = r.p.f.zl;
-                sa->m[threadIdx.x] = real ? r.m : 0.0f;
-                sa->vx[threadIdx.x] = r.vx;
-                sa->vy[threadIdx.x] = r.vy;
-                sa->vz[threadIdx.x] = r.vz;
-                sa->id[threadIdx.x] = r.id;
-                mine = real && r.id >= idlo && r.id <= idhi;
+#pragma unroll
+            for (int q = threadIdx.x; q < NJ; q += NT) {
+                if (q >= nt4) continue;
+                const bool real = q < nt;
+                const G6PredJ r = A.jpred[T.j0 + jt + (real ? q : 0)];
+                sa->xh[q] = r.p.f.xh;
+                sa->yh[q] = r.p.f.yh;
+                sa->zh[q] = r.p.f.zh;
+                sa->xl[q] = r.p.f.xl;
+                sa->yl[q] = r.p.f.yl;
+                sa->zl[q] = r.p.f.zl;
+                sa->m[q] = real ? r.m : 0.0f;
+                sa->vx[q] = r.vx;
+                sa->vy[q] = r.vy;
+                sa->vz[q] = r.vz;
+                sa->id[q] = r.id;
+                mine = mine || (real && r.id >= idlo && r.id <= idhi);
             }
         } else {
             if (threadIdx.x < nt) {
@@ -818,15 +853,17 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
             if constexpr (USE_JP) {
                 // a full tile that cannot hold one of the task's i runs every fold block with a
                 // constant trip count (FULL); self and partial tiles with the run-time count
-                constexpr bool FULL = !SELF && NT % G6_FOLD == 0;
-                for (int j0 = 0; j0 < (FULL ? NT : nt4); j0 += G6_FOLD) {
-                    const int j1 = FULL ? j0 + G6_FOLD : min(j0 + G6_FOLD, nt4);
+                // (a lane of a split tile sees 64 of its j, one block)
+                constexpr int FOLD = JL > 1 ? NJ : G6_FOLD;
+                constexpr bool FULL = !SELF && NJ % FOLD == 0;
+                for (int j0 = 0; j0 < (FULL ? NJ : nt4); j0 += FOLD) {
+                    const int j1 = FULL ? j0 + FOLD : min(j0 + FOLD, nt4);
                     G6Acc2 a[IPT];
                     const float2 z2 = make_float2(0.f, 0.f);
 #pragma unroll
                     for (int k = 0; k < IPT; k++) a[k] = G6Acc2{z2, z2, z2, z2, z2, z2, {0.f, 0.f}};
 #pragma unroll 1
-                    for (int j = j0; j < j1; j += 4) {
+                    for (int j = j0 + 4 * (JL > 1 ? jl : 0); j < j1; j += 4 * JL) {
                         const float4 XH = *reinterpret_cast<const float4*>(&sa->xh[j]);
                         const float4 YH = *reinterpret_cast<const float4*>(&sa->yh[j]);
                         const float4 ZH = *reinterpret_cast<const float4*>(&sa->zh[j]);
@@ -839,8 +876,11 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
                         const float4 VZ = *reinterpret_cast<const float4*>(&sa->vz[j]);
                         int4 ID = make_int4(0, 0, 0, 0);
                         if constexpr (SELF) ID = *reinterpret_cast<const int4*>(&sa->id[j]);
+                        float tq[IPT];   // the running key minimum (QUADMIN: with this j-quad)
+#pragma unroll
+                        for (int k = 0; k < IPT; k++) tq[k] = QUADMIN ? kmin[k] : tmin[k];
                         if constexpr (JP == 2 && IPT == 2) {
-                            g6_jquad2<NN, SELF>(XH, YH, ZH, XL, YL, ZL, M, VX, VY, VZ, ID, IP, A.eps2, a, tmin);
+                            g6_jquad2<NN, SELF>(XH, YH, ZH, XL, YL, ZL, M, VX, VY, VZ, ID, IP, A.eps2, a, tq);
                         } else {
 #pragma unroll
                         for (int k = 0; k < IPT; k++) {
@@ -849,14 +889,25 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
                                                make_float2(YL.x, YL.y), make_float2(ZL.x, ZL.y),
                                                make_float2(M.x, M.y), make_float2(VX.x, VX.y),
                                                make_float2(VY.x, VY.y), make_float2(VZ.x, VZ.y),
-                                               make_int2(ID.x, ID.y), IP[k], A.eps2, a[k], tmin[k]);
+                                               make_int2(ID.x, ID.y), IP[k], A.eps2, a[k], tq[k]);
                             g6_jpair<NN, SELF>(make_float2(XH.z, XH.w), make_float2(YH.z, YH.w),
                                                make_float2(ZH.z, ZH.w), make_float2(XL.z, XL.w),
                                                make_float2(YL.z, YL.w), make_float2(ZL.z, ZL.w),
                                                make_float2(M.z, M.w), make_float2(VX.z, VX.w),
                                                make_float2(VY.z, VY.w), make_float2(VZ.z, VZ.w),
-                                               make_int2(ID.z, ID.w), IP[k], A.eps2, a[k], tmin[k]);
+                                               make_int2(ID.z, ID.w), IP[k], A.eps2, a[k], tq[k]);
                         }
+                        }
+                        if constexpr (NN) {
+#pragma unroll
+                            for (int k = 0; k < IPT; k++) {
+                                if constexpr (QUADMIN) {
+                                    kadr[k] = tq[k] < kmin[k] ? jt + j : kadr[k];
+                                    kmin[k] = tq[k];
+                                } else {
+                                    tmin[k] = tq[k];
+                                }
+                            }
                         }
                     }
 #pragma unroll
@@ -946,7 +997,7 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
                 }
             }
         };
-        if (USE_JP ? (self_tile || nt4 != NT) : self_tile) run_tile(BoolC<true>{});
+        if (USE_JP ? (self_tile || nt4 != NJ) : self_tile) run_tile(BoolC<true>{});
         else run_tile(BoolC<false>{});
 
         if constexpr (TILEMIN) {
@@ -975,10 +1026,10 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
             } else if (li < T.ni && ktile[k] >= 0) {
                 if constexpr (USE_JP) {
                     const G6I P = A.ipart[T.i0 + li];
-                    kadr[k] = g6_rescan<FF>(A.jpred, T.j0 + ktile[k], min(NT, T.nj - ktile[k]), P.p, P.id, A.eps2,
+                    kadr[k] = g6_rescan<FF>(A.jpred, T.j0 + ktile[k], min(NJ, T.nj - ktile[k]), P.p, P.id, A.eps2,
                                             kmin[k]);
                 } else {
-                    kadr[k] = g6_rescan<FF>(A.jpred, T.j0 + ktile[k], min(NT, T.nj - ktile[k]), pi[k], idi[k],
+                    kadr[k] = g6_rescan<FF>(A.jpred, T.j0 + ktile[k], min(NJ, T.nj - ktile[k]), pi[k], idi[k],
                                             A.eps2, kmin[k]);
                 }
             }
@@ -986,9 +1037,11 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
     }
     if constexpr (USE_JP) {
 #pragma unroll
-        for (int k = 0; k < IPT; k++)
+        for (int k = 0; k < IPT; k++) {
+            if (QUADMIN && kadr[k] >= 0) kadr[k] += T.j0;
 #pragma unroll
             for (int c = 0; c < 7; c++) S[k][c] = Ssh[(k * 7 + c) * NT + threadIdx.x];
+        }
     }
 
     G6Out* dst_row = (T.group < 0) ? nullptr : A.partial + (size_t)T.slot * A.itile;
@@ -1010,8 +1063,12 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
         }
         int li = slot + k * ISL;
         if (li >= T.ni) continue;
-        if (dst_row) dst_row[li] = o;
-        else A.out[T.i0 + li] = g6_finish(o);
+        if (dst_row) {
+            dst_row[li] = o;
+        } else {
+            if constexpr (QUADMIN) o.jadr = g6_quad_lookup<FF>(A, T.i0 + li, o.key, o.jadr);
+            A.out[T.i0 + li] = g6_finish(o);
+        }
     }
 }
 
@@ -1026,11 +1083,11 @@ constexpr int g6_min_ctas() {
 }
 
 template <int NT, int IPT, int JL, bool FF, bool NN, bool NBL, int JP = 0>
-__global__ void __launch_bounds__(NT, g6_min_ctas<NT, IPT, JP && FF && !NBL && (IPT == 2 || IPT == 4) && JL == 1>())
+__global__ void __launch_bounds__(NT, g6_min_ctas<NT, IPT, g6_uses_jp<IPT, FF, NBL, JP>()>())
     g6_kernel(const G6Args A) {
+    constexpr bool USE_JP = g6_uses_jp<IPT, FF, NBL, JP>();
     // j tile during the loop, per-thread results (G6Out) after it
-    __shared__ __align__(16) unsigned char
-        smem[g6_smem_bytes<NT, IPT, JP && FF && !NBL && (IPT == 2 || IPT == 4) && JL == 1>()];
+    __shared__ __align__(16) unsigned char smem[g6_smem_bytes<NT, IPT, USE_JP, g6_tile_j<NT, JL, USE_JP>()>()];
     __shared__ int s_task, s_flag;
 
     for (bool first = true;; first = false) {
@@ -1042,6 +1099,7 @@ __global__ void __launch_bounds__(NT, g6_min_ctas<NT, IPT, JP && FF && !NBL && (
         const Group G = A.groups ? A.groups[T.group] : regular_group(A, T.group);
         double2* W = reinterpret_cast<double2*>(smem);
         const int B = bundle_size(G.nchunk, A.bundle_counters != nullptr);
+        G6Out* const out = A.out + G.i0;
         if (B < G.nchunk) {
             // two levels: the last CTA of each bundle of B consecutive chunks sums the bundle's
             // rows into the bundle's first row, the last bundle of the group sums those
@@ -1053,12 +1111,15 @@ __global__ void __launch_bounds__(NT, g6_min_ctas<NT, IPT, JP && FF && !NBL && (
             reduce_rows<NT>(row0, (size_t)A.itile, nbk, 0, 4 * G.ni, row0, false, W);
             const int nb = (G.nchunk + B - 1) / B;
             if (!group_arrive(A.group_counters, T.group, nb, &s_flag)) continue;
-            reduce_rows<NT>(A.partial + (size_t)G.slot0 * A.itile, (size_t)B * A.itile, nb, 0, 4 * G.ni, A.out + G.i0, true,
-                            W);
+            reduce_rows<NT>(A.partial + (size_t)G.slot0 * A.itile, (size_t)B * A.itile, nb, 0, 4 * G.ni, out, true, W);
         } else {
             if (!group_arrive(A.group_counters, T.group, G.nchunk, &s_flag)) continue;
-            reduce_rows<NT>(A.partial + (size_t)G.slot0 * A.itile, (size_t)A.itile, G.nchunk, 0, 4 * G.ni, A.out + G.i0,
-                            true, W);
+            reduce_rows<NT>(A.partial + (size_t)G.slot0 * A.itile, (size_t)A.itile, G.nchunk, 0, 4 * G.ni, out, true, W);
+        }
+        if constexpr (NN && g6_quad_min<IPT, FF, NBL, JP>()) {
+            __syncthreads();
+            for (int r = threadIdx.x; r < G.ni; r += NT)
+                out[r].jadr = g6_quad_lookup<FF>(A, G.i0 + r, key_in(out[r].key), out[r].jadr);
         }
     }
 }
