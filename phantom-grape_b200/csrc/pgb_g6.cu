@@ -1648,6 +1648,10 @@ bool hm_alloc(pgb6_hermite* H) {
     H->P.jrk = b + 13 * n;
     H->nseg = (int)((n + HM_SEG - 1) / HM_SEG);
     H->grid = hm_grid(H->ff);
+    if (H->grid < HM_MAXSEG / HM_OWN) {
+        raise(g_err, LIB, PGB_ERR_CAPACITY, "pgb6_hermite_create: %d co-resident CTAs are too few", H->grid);
+        return false;
+    }
     // partial rows: at most (grid + i-tiles) rows of at most 512 entries; force tasks: at most
     // grid + i-tiles of at least 16
     const long long part_cap = (long long)H->grid * 512 + (long long)n + 512;
@@ -1655,18 +1659,18 @@ bool hm_alloc(pgb6_hermite* H) {
     size_t off = 0;
     const size_t o_hdr = off;
     off = align256(off + sizeof(HmClock));
-    const size_t o_sync = off;
-    off = align256(off + sizeof(HmSync) + sizeof(unsigned) * (size_t)H->grid * HM_ARRIVE_STRIDE);
-    const size_t o_gmin = off;
-    off = align256(off + 3 * sizeof(unsigned long long));
-    const size_t o_bmin = off;
-    off = align256(off + sizeof(unsigned long long) * 2 * H->nseg);
-    const size_t o_bcnt = off;
-    off = align256(off + sizeof(int) * 2 * H->nseg);
+    const size_t o_rec = off;
+    off = align256(off + sizeof(HmWord) * HM_RSLOTS * H->nseg);
+    const size_t o_list = off;
+    off = align256(off + (size_t)HM_RSLOTS * H->nseg * HM_SEG);
+    const size_t o_ack = off;
+    off = align256(off + sizeof(unsigned) * (size_t)H->grid);
+    const size_t o_sums = off;
+    off = align256(off + sizeof(HmWord) * HM_SUMW * HM_SMALL * (size_t)H->grid);
     const size_t o_sflag = off;
     off = align256(off + sizeof(unsigned) * H->nseg);
     const size_t o_tflag = off;
-    off = align256(off + sizeof(unsigned) * (size_t)task_cap);
+    off = align256(off + sizeof(unsigned) * ((size_t)task_cap + H->grid));
     const size_t o_act = off;
     off = align256(off + sizeof(int) * n);
     const size_t o_irec = off;
@@ -1682,10 +1686,11 @@ bool hm_alloc(pgb6_hermite* H) {
     PGB_CUDA_OR(g_err, LIB, H->work.reserve(off), return false);
     unsigned char* w = H->work.p;
     H->W.clk = (HmClock*)(w + o_hdr);
-    H->W.sync = (HmSync*)(w + o_sync);
-    H->W.gmin = (unsigned long long*)(w + o_gmin);
-    H->W.bmin = (unsigned long long*)(w + o_bmin);
-    H->W.bcnt = (int*)(w + o_bcnt);
+    H->W.rec = (HmWord*)(w + o_rec);
+    H->W.seg_list = w + o_list;
+    H->W.ack = (unsigned*)(w + o_ack);
+    H->W.sums = (HmWord*)(w + o_sums);
+    H->W.chunks = H->grid;
     H->W.seg_flag = (unsigned*)(w + o_sflag);
     H->W.task_flag = (unsigned*)(w + o_tflag);
     H->W.task_cap = task_cap;
@@ -1696,12 +1701,8 @@ bool hm_alloc(pgb6_hermite* H) {
     H->W.partial = (G6Out*)(w + o_part);
     H->W.part_cap = part_cap;
     H->energy = (double*)(w + o_en);
-    // clock, barrier and flags zero; the step numbers that tag the flags start at 1
+    // clock, records and flags zero; the step numbers that tag them start at 1
     PGB_CUDA_OR(g_err, LIB, cudaMemsetAsync(w, 0, o_act, H->s), return false);
-    const unsigned first_step = 1;
-    PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(&H->W.sync->step, &first_step, sizeof first_step, cudaMemcpyHostToDevice,
-                                            H->s), return false);
-    PGB_CUDA_OR(g_err, LIB, cudaStreamSynchronize(H->s), return false);
     return true;
 }
 
@@ -1711,7 +1712,7 @@ bool hm_sync_clock(pgb6_hermite* H) {
                 return false);
     PGB_CUDA_OR(g_err, LIB, cudaStreamSynchronize(H->s), return false);
     if (H->clk.err) {
-        raise(g_err, LIB, PGB_ERR_DEVICE, "hermite: a grid barrier of the step kernel timed out");
+        raise(g_err, LIB, PGB_ERR_DEVICE, "hermite: a wait of the step kernel timed out");
         return false;
     }
     return true;
@@ -1728,6 +1729,10 @@ bool hm_launch(pgb6_hermite* H, bool startup, double tend, int max_steps) {
     R.eta_s = H->eta_s;
     R.dtmax = H->dtmax;
     R.tend = tend;
+    // the clock of the last launch, which has been read back (hm_sync_clock); every step counted one
+    R.step0 = 1u + (unsigned)H->clk.bsteps;
+    R.time0 = H->clk.time;
+    R.t_mod0 = H->clk.t_mod;
     R.startup = startup ? 1 : 0;
     R.max_steps = max_steps;
     R.nseg = H->nseg;
@@ -1735,6 +1740,9 @@ bool hm_launch(pgb6_hermite* H, bool startup, double tend, int max_steps) {
     // to sum; N = 16384 block steps: 64 -> 114, 128 -> 120, 256 -> 123, 512 -> 108 Gint/s)
     static const int minj = env_int("PGB_HM_MINJ", 256, 16, 1 << 20);
     R.minj = minj;
+    // hm_shape's chunk count of a single i-tile of at most HM_SMALL (its buffers never limit that)
+    R.nch1 = std::min(H->grid, std::max(1, H->n / minj));
+    R.dtinv = 1.0 / H->dtmax;
     void* args[] = {&R};
     const void* fn = H->ff ? (const void*)hm_run_kernel<true> : (const void*)hm_run_kernel<false>;
     PGB_CUDA_OR(g_err, LIB, cudaLaunchCooperativeKernel(fn, dim3(H->grid), dim3(HM_NT), args, 0, H->s),
