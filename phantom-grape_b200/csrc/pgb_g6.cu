@@ -1648,7 +1648,7 @@ bool hm_alloc(pgb6_hermite* H) {
     H->P.jrk = b + 13 * n;
     H->nseg = (int)((n + HM_SEG - 1) / HM_SEG);
     H->grid = hm_grid(H->ff);
-    if (H->grid < HM_MAXSEG / HM_OWN) {
+    if (H->nseg > HM_OWN * H->grid) {
         raise(g_err, LIB, PGB_ERR_CAPACITY, "pgb6_hermite_create: %d co-resident CTAs are too few", H->grid);
         return false;
     }
