@@ -211,9 +211,10 @@ inline SmallShape small_shape(int ni) {
 // CTA, where the 33 clusters of 8 left 32 (the others, with two, set the call's time): the
 // 48 x 65536 call 27.2 -> 26.6 us, 48 x 16384 23.0 -> 19.7 us
 constexpr int SMALL_CL = 4;
+constexpr int SMALL_WORDS = sizeof(G6Out) / 4;   // host words of a result
 
 template <int ISL, int JL, bool FF, bool NN, bool NBL>
-cudaError_t small_launch(int grid, int cl, const G6SmallArgs& a, const G6IBlock& ib, cudaStream_t s,
+cudaError_t small_launch(int grid, int cl, const G6SmallArgs& a, const G6I* irec, cudaStream_t s,
                          int* max_clusters) {
     auto kern = g6_small_kernel<ISL, JL, FF, NN, NBL>;
     cudaLaunchConfig_t cfg = {};
@@ -229,32 +230,34 @@ cudaError_t small_launch(int grid, int cl, const G6SmallArgs& a, const G6IBlock&
     cfg.attrs = at;
     cfg.numAttrs = 1;
     if (max_clusters) return cudaOccupancyMaxActiveClusters(max_clusters, (void*)kern, &cfg);
+    G6IBlock<ISL> ib;
+    std::memcpy(ib.rec, irec, (size_t)a.ni * sizeof(G6I));
     return cudaLaunchKernelEx(&cfg, kern, a, ib);
 }
 
 template <int ISL, int JL, bool FF>
 cudaError_t small_launch_nn(bool nn, bool nbl, int grid, int cl, const G6SmallArgs& a,
-                            const G6IBlock& ib, cudaStream_t s, int* mc) {
-    if (nn && nbl) return small_launch<ISL, JL, FF, true, true>(grid, cl, a, ib, s, mc);
-    if (nn) return small_launch<ISL, JL, FF, true, false>(grid, cl, a, ib, s, mc);
-    if (nbl) return small_launch<ISL, JL, FF, false, true>(grid, cl, a, ib, s, mc);
-    return small_launch<ISL, JL, FF, false, false>(grid, cl, a, ib, s, mc);
+                            const G6I* irec, cudaStream_t s, int* mc) {
+    if (nn && nbl) return small_launch<ISL, JL, FF, true, true>(grid, cl, a, irec, s, mc);
+    if (nn) return small_launch<ISL, JL, FF, true, false>(grid, cl, a, irec, s, mc);
+    if (nbl) return small_launch<ISL, JL, FF, false, true>(grid, cl, a, irec, s, mc);
+    return small_launch<ISL, JL, FF, false, false>(grid, cl, a, irec, s, mc);
 }
 
 template <bool FF>
 cudaError_t small_launch_ff(SmallShape sh, bool nn, bool nbl, int grid, int cl, const G6SmallArgs& a,
-                            const G6IBlock& ib, cudaStream_t s, int* mc) {
-    if (sh.isl == 16) return small_launch_nn<16, 32, FF>(nn, nbl, grid, cl, a, ib, s, mc);
-    if (sh.isl == 32) return small_launch_nn<32, 16, FF>(nn, nbl, grid, cl, a, ib, s, mc);
-    if (sh.isl == 48) return small_launch_nn<48, 10, FF>(nn, nbl, grid, cl, a, ib, s, mc);
-    return small_launch_nn<64, 8, FF>(nn, nbl, grid, cl, a, ib, s, mc);
+                            const G6I* irec, cudaStream_t s, int* mc) {
+    if (sh.isl == 16) return small_launch_nn<16, 32, FF>(nn, nbl, grid, cl, a, irec, s, mc);
+    if (sh.isl == 32) return small_launch_nn<32, 16, FF>(nn, nbl, grid, cl, a, irec, s, mc);
+    if (sh.isl == 48) return small_launch_nn<48, 10, FF>(nn, nbl, grid, cl, a, irec, s, mc);
+    return small_launch_nn<64, 8, FF>(nn, nbl, grid, cl, a, irec, s, mc);
 }
 
 // Launch (mc == nullptr) or query the co-resident clusters of cl CTAs (into *mc).
 cudaError_t small_kernel(SmallShape sh, bool ff, bool nn, bool nbl, int grid, int cl, const G6SmallArgs& a,
-                         const G6IBlock& ib, cudaStream_t s, int* mc) {
-    return ff ? small_launch_ff<true>(sh, nn, nbl, grid, cl, a, ib, s, mc)
-              : small_launch_ff<false>(sh, nn, nbl, grid, cl, a, ib, s, mc);
+                         const G6I* irec, cudaStream_t s, int* mc) {
+    return ff ? small_launch_ff<true>(sh, nn, nbl, grid, cl, a, irec, s, mc)
+              : small_launch_ff<false>(sh, nn, nbl, grid, cl, a, irec, s, mc);
 }
 
 // Chunks (= CTAs, all co-resident) and cluster size of a small call over nj j-records: at least
@@ -265,9 +268,8 @@ void small_grid(SmallShape sh, bool ff, bool nn, bool nbl, int nj, int& grid, in
     int& mc = cache[v][ff][nn][nbl];
     if (!mc) {
         G6SmallArgs a{};
-        G6IBlock ib{};
         int n = 0;
-        if (small_kernel(sh, ff, nn, nbl, SMALL_CL, SMALL_CL, a, ib, nullptr, &n) != cudaSuccess || n < 1) {
+        if (small_kernel(sh, ff, nn, nbl, SMALL_CL, SMALL_CL, a, nullptr, nullptr, &n) != cudaSuccess || n < 1) {
             cudaGetLastError();
             n = sm_count(g_device) / SMALL_CL;
         }
@@ -282,6 +284,7 @@ void small_grid(SmallShape sh, bool ff, bool nn, bool nbl, int nj, int& grid, in
     cl = 1;
     while (cl < SMALL_CL && cl * 2 <= want) cl *= 2;
     grid = want / cl * cl;
+    if (grid == SMALL_CL_MAX) cl = grid;   // one cluster: no rows of partial sums in memory
 }
 
 // Relative-coordinate arithmetic of the library's own calls: double-float (default) or FP64
@@ -431,10 +434,12 @@ struct State {
     std::vector<int> dirty;
     std::vector<unsigned char> dirty_flag;
     bool all_dirty = true;
-    HostBuf<G6Ptcl> sbuf;   // packed dirty records
-    HostBuf<int> sidx;      // their addresses
-    DevBuf<G6Ptcl> sbuf_d;
-    DevBuf<int> sidx_d;
+    HostBuf<G6Ptcl> sbuf;   // mapped: packed dirty records
+    HostBuf<int> sidx;      // mapped: their addresses
+    // the stream may still read jh, sbuf or sidx (g6calc_firsthalf does not wait for its upload)
+    bool uploading = false;
+    G6Ptcl* sbuf_dev = nullptr;
+    int* sidx_dev = nullptr;
     double ti = 0.0;
     int predict_flag = 0;
     HostBuf<G6I> ibuf;
@@ -442,17 +447,20 @@ struct State {
     G6Out* outh_dev = nullptr;            // its device address (looked up once per allocation)
     const G6Out* outh_seen = nullptr;     // the allocation outh_dev belongs to
     DevBuf<int> pcnt;       // self-resetting counters of the parameter-block launches
-    G6IBlock iblk;  // their i-records
     DevBuf<G6Out> spart;    // cluster rows of the small-call kernel
-    HostBuf<unsigned> flags;  // mapped completion flags of the small-call kernel
-    unsigned* flags_dev = nullptr;
-    unsigned seq = 0;         // sequence number of the last flagged call
-    int wait_flags = 0;       // flags the next wait_results() polls (0: synchronise the stream)
+    HostBuf<uint2> words;     // mapped: the small-call kernel's results, (value, call number) words
+    uint4* words_dev = nullptr;
+    unsigned seq = 0;         // number of the last small call
+    bool wait_words = false;  // the call's results come in `words` (else in outh, after the stream)
+    HostBuf<uint2> nbw;       // mapped: its neighbour lists, [ni][nbmax + 1] of (value, call number)
+    uint2* nbw_dev = nullptr;
+    bool nbc_zero = false;    // the list counts nbc_d are zero
     Stager<G6I, G6Out> st;
     // neighbour lists of the last lasthalf*n call
     DevBuf<int> nbc_d, nbl_d;
     HostBuf<int> nbc_h, nbl_h;
-    std::vector<std::vector<int>> nblists;
+    std::vector<int> nbids;   // one after another, list i from nboff[i]
+    std::vector<size_t> nboff;
     std::vector<int> nbcounts;
     // device-time accounting of the drop-in calls (pgb6_set_call_timing): CUDA events around the
     // j-update + prediction of g6calc_firsthalf and the force launch of g6calc_lasthalf*
@@ -472,6 +480,14 @@ bool init_state() {
     return true;
 }
 
+// Before the host changes what an upload reads.
+bool wait_upload() {
+    if (!S.uploading) return true;
+    PGB_CUDA_OR(g_err, LIB, cudaStreamSynchronize(S.stream), return false);
+    S.uploading = false;
+    return true;
+}
+
 bool grow_j(int need) {
     if (need > jmemsize()) {
         raise(g_err, LIB, PGB_ERR_CAPACITY, "j-memory overflow: address %d >= jmemsize %d", need - 1, jmemsize());
@@ -481,6 +497,7 @@ bool grow_j(int need) {
     int cap = S.jcap ? S.jcap : 8192;
     while (cap < need) cap *= 2;
     if (cap > jmemsize()) cap = jmemsize();
+    if (!wait_upload()) return false;
     PGB_CUDA_OR(g_err, LIB, S.jh.reserve(cap, true), return false);
     std::memset((void*)(S.jh.p + S.jcap), 0, (size_t)(cap - S.jcap) * sizeof(G6Ptcl));
     S.dirty_flag.resize(cap, 0);
@@ -500,37 +517,69 @@ void mark_dirty(int padr) {
     }
 }
 
-// Upload the j-memory changes: the contiguous dirty range, or, when the changed records are
-// sparse in it (a block step's active set), only those records plus a scatter on the device.
-bool flush_j() {
-    if (S.jdirty_hi <= S.jdirty_lo) return true;
-    PGB_CUDA_OR(g_err, LIB, S.jd.reserve(S.jcap), return false);
-    size_t lo = S.jdirty_lo, range = (size_t)(S.jdirty_hi - S.jdirty_lo), n = S.dirty.size();
-    if (!S.all_dirty && n * 4 < range) {
-        PGB_CUDA_OR(g_err, LIB, S.sbuf.reserve(n), return false);
-        PGB_CUDA_OR(g_err, LIB, S.sidx.reserve(n), return false);
-        PGB_CUDA_OR(g_err, LIB, S.sbuf_d.reserve(n), return false);
-        PGB_CUDA_OR(g_err, LIB, S.sidx_d.reserve(n), return false);
-        for (size_t k = 0; k < n; k++) {
-            S.sbuf.p[k] = S.jh.p[S.dirty[k]];
-            S.sidx.p[k] = S.dirty[k];
-        }
-        PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(S.sbuf_d.p, S.sbuf.p, n * sizeof(G6Ptcl), cudaMemcpyHostToDevice,
-                                                S.stream), return false);
-        PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(S.sidx_d.p, S.sidx.p, n * sizeof(int), cudaMemcpyHostToDevice,
-                                                S.stream), return false);
-        g6_scatter_kernel<<<(int)((n + 255) / 256), 256, 0, S.stream>>>(S.sbuf_d.p, S.sidx_d.p, (int)n, S.jcap,
-                                                                         S.jd.p);
-        PGB_CUDA_OR(g_err, LIB, cudaGetLastError(), return false);
-    } else {
-        PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(S.jd.p + lo, S.jh.p + lo, range * sizeof(G6Ptcl),
-                                                cudaMemcpyHostToDevice, S.stream), return false);
+// Room for `want` items in a mapped buffer, and its device address (looked up when it is allocated).
+template <class T, class D>
+bool reserve_mapped(HostBuf<T>& b, size_t want, D*& dev) {
+    const T* old = b.p;
+    PGB_CUDA_OR(g_err, LIB, b.reserve(want, false, cudaHostAllocPortable | cudaHostAllocMapped), return false);
+    if (b.p != old || !dev) {
+        dev = nullptr;
+        PGB_CUDA_OR(g_err, LIB, cudaHostGetDevicePointer((void**)&dev, b.p, 0), return false);
     }
-    for (int a : S.dirty) S.dirty_flag[a] = 0;
-    S.dirty.clear();
-    S.all_dirty = false;
-    S.jdirty_lo = 1 << 30;
-    S.jdirty_hi = 0;
+    return true;
+}
+
+// Upload the j-memory changes and predict j-records [0, nj) to the set time: the contiguous dirty
+// range by a copy, or, when the changed records are sparse in it (a block step's active set), only
+// those, which the device reads from mapped host memory -- up to G6_UPD_MAX in the prediction's
+// own launch, more by a scatter before it (its address list would make the launch's parameters grow;
+// two copies and a scatter instead: 47 against 36 us a call of 7 i with 7 of 1024 records sent).
+bool launch_update(int nj) {
+    PGB_CUDA_OR(g_err, LIB, S.pred.reserve(S.jcap), return false);
+    const bool dirty = S.jdirty_hi > S.jdirty_lo;
+    const size_t n = S.dirty.size();
+    const bool sparse = dirty && !S.all_dirty && n * 4 < (size_t)(S.jdirty_hi - S.jdirty_lo);
+    const bool fused = sparse && n <= (size_t)G6_UPD_MAX;
+    G6Ptcl* rec_d = nullptr;
+    if (dirty) {
+        PGB_CUDA_OR(g_err, LIB, S.jd.reserve(S.jcap), return false);
+        if (!wait_upload()) return false;
+        S.uploading = true;
+    }
+    if (sparse) {
+        if (!reserve_mapped(S.sbuf, n, S.sbuf_dev)) return false;
+        rec_d = S.sbuf_dev;
+        for (size_t k = 0; k < n; k++) S.sbuf.p[k] = S.jh.p[S.dirty[k]];
+    }
+    if (fused) {
+        G6Update U;
+        U.rec = rec_d;
+        U.n = (int)n;
+        std::memcpy(U.idx, S.dirty.data(), n * sizeof(int));
+        const int top = std::max(nj, S.jdirty_hi);
+        g6_update_predict_kernel<<<(top + 255) / 256, 256, 0, S.stream>>>(S.jd.p, S.jcap, U, nj, S.ti, S.pred.p,
+                                                                          dx_ff());
+    } else {
+        if (sparse) {
+            if (!reserve_mapped(S.sidx, n, S.sidx_dev)) return false;
+            std::memcpy(S.sidx.p, S.dirty.data(), n * sizeof(int));
+            g6_scatter_kernel<<<(int)((n + 255) / 256), 256, 0, S.stream>>>(rec_d, S.sidx_dev, (int)n, S.jcap, S.jd.p);
+            PGB_CUDA_OR(g_err, LIB, cudaGetLastError(), return false);
+        } else if (dirty) {
+            const size_t lo = S.jdirty_lo, range = (size_t)(S.jdirty_hi - S.jdirty_lo);
+            PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(S.jd.p + lo, S.jh.p + lo, range * sizeof(G6Ptcl),
+                                                    cudaMemcpyHostToDevice, S.stream), return false);
+        }
+        g6_predict_kernel<<<(nj + 255) / 256, 256, 0, S.stream>>>(S.jd.p, nj, S.ti, S.pred.p, dx_ff());
+    }
+    PGB_CUDA_OR(g_err, LIB, cudaGetLastError(), return false);
+    if (dirty) {
+        for (int a : S.dirty) S.dirty_flag[a] = 0;
+        S.dirty.clear();
+        S.all_dirty = false;
+        S.jdirty_lo = 1 << 30;
+        S.jdirty_hi = 0;
+    }
     return true;
 }
 
@@ -552,21 +601,28 @@ bool time_add() {
     return true;
 }
 
+// The upload and prediction of g6calc_firsthalf, left running: g6calc_lasthalf* follows on the same
+// stream and waits for both, and what would change the upload's source waits first (wait_upload).  Waiting
+// here cost the call of 48 i against 65536 j 42 -> 31.5 us.  (The prediction inside the force kernel
+// instead of its own launch is no faster: it then starts with the force, not while the host prepares it.)
 bool flush_and_predict(int nj) {
     if (nj <= 0) return true;
-    if (!grow_j(nj) || !time_mark(0) || !flush_j()) return false;
-    PGB_CUDA_OR(g_err, LIB, S.pred.reserve(S.jcap), return false);
-    g6_predict_kernel<<<(nj + 255) / 256, 256, 0, S.stream>>>(S.jd.p, nj, S.ti, S.pred.p, dx_ff());
-    PGB_CUDA_OR(g_err, LIB, cudaGetLastError(), return false);
-    if (!time_mark(1)) return false;
-    // j-memory is read asynchronously from the pinned mirror: later set_j calls wait for it
-    PGB_CUDA_OR(g_err, LIB, cudaStreamSynchronize(S.stream), return false);
+    if (!grow_j(nj) || !time_mark(0) || !launch_update(nj) || !time_mark(1)) return false;
     return time_add();
 }
 
-// The small-call path: one launch of the cluster kernel (i-records in its parameter block),
-// results into the mapped buffer; the call is one launch and one stream synchronisation.
-bool run_small(int nj, int ni, float eps2, bool nn, bool nbl, G6Out* out_dev) {
+// Shared memory of g6_nb_sort_kernel: the power of two at or above nbmax entries.
+size_t nb_sort_smem() {
+    size_t p = 1;
+    while (p < (size_t)nbmax()) p <<= 1;
+    return p * sizeof(int);
+}
+
+// The small-call path: one launch of the cluster kernel (i-records in its parameter block) and, with
+// neighbour lists, one that sorts them; results and lists come as words in mapped buffers, which the
+// host takes as they arrive (33 i against 20011 j with lists: 114 -> 61 us, 27 of them the caller's reading
+// of the lists).
+bool run_small(int nj, int ni, float eps2, bool nn, bool nbl) {
     const bool ff = dx_ff();
     const SmallShape sh = small_shape(ni);
     int grid = 1, cl = 1;
@@ -583,55 +639,79 @@ bool run_small(int nj, int ni, float eps2, bool nn, bool nbl, G6Out* out_dev) {
     a.nj = nj;
     a.partial = S.spart.p;
     a.counter = S.pcnt.p;
-    a.out = out_dev;
     a.nb_count = nullptr;
     a.nb_list = nullptr;
     a.nb_maxlen = nbmax();
     if (nbl) {
-        PGB_CUDA_OR(g_err, LIB, S.nbc_d.reserve(ni), return false);
+        if (!S.nbc_zero || !S.nbc_d.p) {
+            PGB_CUDA_OR(g_err, LIB, S.nbc_d.reserve(G6_SMALL_MAXI), return false);
+            PGB_CUDA_OR(g_err, LIB, cudaMemsetAsync(S.nbc_d.p, 0, G6_SMALL_MAXI * sizeof(int), S.stream), return false);
+        }
         PGB_CUDA_OR(g_err, LIB, S.nbl_d.reserve((size_t)ni * nbmax()), return false);
-        PGB_CUDA_OR(g_err, LIB, cudaMemsetAsync(S.nbc_d.p, 0, (size_t)ni * sizeof(int), S.stream), return false);
         a.nb_count = S.nbc_d.p;
         a.nb_list = S.nbl_d.p;
     }
-    // completion flags (mapped host memory, one per word slice of the final stage)
-    a.done = nullptr;
-    a.seq = 0;
-    if (!nbl) {
-        if (!S.flags.p) {
-            PGB_CUDA_OR(g_err, LIB, S.flags.reserve(SMALL_CL, false, cudaHostAllocPortable | cudaHostAllocMapped),
-                        return false);
-            std::memset((void*)S.flags.p, 0, SMALL_CL * sizeof(unsigned));
-            PGB_CUDA_OR(g_err, LIB, cudaHostGetDevicePointer((void**)&S.flags_dev, S.flags.p, 0), return false);
-        }
-        a.done = S.flags_dev;
-        a.seq = ++S.seq;
-        if (a.seq == 0) a.seq = ++S.seq;   // 0 is the flags' initial value
-        S.wait_flags = cl;
+    // no word of the buffers carries the number of a call to come: they start with the number of a call
+    // that is over, and are cleared when the numbers start again
+    const size_t nword = SMALL_WORDS * G6_SMALL_MAXI, nnb = (size_t)G6_SMALL_MAXI * (nbmax() + 1);
+    const bool fresh = !S.words.p, fresh_nb = nbl && !S.nbw.p;
+    if (!reserve_mapped(S.words, nword, S.words_dev)) return false;
+    if (nbl && !reserve_mapped(S.nbw, nnb, S.nbw_dev)) return false;
+    const bool wrap = ++S.seq == 0;
+    if (wrap) S.seq = 1;
+    if (fresh || wrap) std::memset((void*)S.words.p, 0, sizeof(uint2) * nword);
+    if (fresh_nb || (wrap && S.nbw.p)) std::memset((void*)S.nbw.p, 0, sizeof(uint2) * nnb);
+    a.words = S.words_dev;
+    a.seq = S.seq;
+    S.wait_words = true;
+    PGB_CUDA_OR(g_err, LIB, small_kernel(sh, ff, nn, nbl, grid, cl, a, S.ibuf.p, S.stream, nullptr), return false);
+    if (nbl) {
+        S.nbc_zero = false;
+        g6_nb_sort_kernel<<<ni, 256, nb_sort_smem(), S.stream>>>(S.nbc_d.p, S.nbl_d.p, nbmax(), S.jd.p, S.nbw_dev,
+                                                                S.seq);
+        PGB_CUDA_OR(g_err, LIB, cudaGetLastError(), return false);
+        S.nbc_zero = true;
     }
-    std::memcpy(S.iblk.rec, S.ibuf.p, (size_t)ni * sizeof(G6I));
-    PGB_CUDA_OR(g_err, LIB, small_kernel(sh, ff, nn, nbl, grid, cl, a, S.iblk, S.stream, nullptr), return false);
     return true;
 }
 
-// Wait for the results of the last call: by its completion flags when it has them (a bounded
-// spin, then the stream synchronisation that reports a failed launch), else the stream.
-bool wait_results() {
-    if (S.wait_flags > 0) {
-        const int n = S.wait_flags;
-        S.wait_flags = 0;
-        const unsigned seq = S.seq;
-        volatile unsigned* f = S.flags.p;
-        auto t0 = std::chrono::steady_clock::now();
-        for (long it = 0;; it++) {
-            bool all = true;
-            for (int k = 0; k < n; k++) all = all && f[k] == seq;
-            if (all) return true;
-            if ((it & 1023) == 1023 && std::chrono::steady_clock::now() - t0 > std::chrono::seconds(5)) break;
-        }
+// Words of a small call as they arrive: take() returns true when it has them all.  A bounded spin, then
+// the stream synchronisation that reports a failed launch.
+template <class Take>
+bool take_words(Take take) {
+    auto t0 = std::chrono::steady_clock::now();
+    for (long it = 0;; it++) {
+        if (take()) return true;
+        if ((it & 1023) == 1023 && std::chrono::steady_clock::now() - t0 > std::chrono::seconds(5)) break;
     }
     PGB_CUDA_OR(g_err, LIB, cudaStreamSynchronize(S.stream), return false);
+    if (take()) return true;
+    raise(g_err, LIB, PGB_ERR_DEVICE, "a call's results did not arrive");
+    return false;
+}
+// Word w's value into v when it carries call number seq.
+template <class T>
+bool take_word(const uint2* w, unsigned seq, T& v) {
+    const unsigned long long x = *(const volatile unsigned long long*)w;
+    if ((unsigned)(x >> 32) != seq) return false;
+    v = (T)(unsigned)x;
     return true;
+}
+
+// Wait for the results of the last call in S.outh: word by word when the call sends words, else the
+// stream.
+bool wait_results(int ni) {
+    if (!S.wait_words) {
+        PGB_CUDA_OR(g_err, LIB, cudaStreamSynchronize(S.stream), return false);
+        return true;
+    }
+    unsigned* out = (unsigned*)S.outh.p;
+    const int n = SMALL_WORDS * ni;
+    int k = 0;
+    return take_words([&] {
+        while (k < n && take_word(S.words.p + k, S.seq, out[k])) k++;
+        return k == n;
+    });
 }
 
 // One drop-in API call: ni i-particles (in S.ibuf) against j-records [0, nj), results into
@@ -646,8 +726,7 @@ bool run_force(int nj, int ni, float eps2, bool nn, bool nbl) {
         PGB_CUDA_OR(g_err, LIB, cudaHostGetDevicePointer((void**)&S.outh_dev, S.outh.p, 0), return false);
         S.outh_seen = S.outh.p;
     }
-    G6Out* out_dev = S.outh_dev;
-    if (ni <= G6_SMALL_MAXI && nj > 0) return run_small(nj, ni, eps2, nn, nbl, out_dev);
+    if (ni <= G6_SMALL_MAXI && nj > 0) return run_small(nj, ni, eps2, nn, nbl);
     const bool ff = dx_ff();
     const int cfg = pick_cfg(ni, nj, ff, nbl);
     const int itile = kernel_info(cfg, ff, nn, nbl).itile;
@@ -671,7 +750,7 @@ bool run_force(int nj, int ni, float eps2, bool nn, bool nbl) {
     a.groups = nullptr;
     a.group_counters = S.st.dgcnt.p;
     a.partial = S.st.dpart.p;
-    a.out = out_dev;
+    a.out = S.outh_dev;
     a.itile = itile;
     a.bundle_counters = S.st.bundle_counters();
     a.nb_count = nullptr;
@@ -682,6 +761,7 @@ bool run_force(int nj, int ni, float eps2, bool nn, bool nbl) {
     a.reg_nch = nch;
     a.jn = nj;
     if (nbl) {
+        S.nbc_zero = false;
         PGB_CUDA_OR(g_err, LIB, S.nbc_d.reserve(ni), return false);
         PGB_CUDA_OR(g_err, LIB, S.nbl_d.reserve((size_t)ni * nbmax()), return false);
         PGB_CUDA_OR(g_err, LIB, cudaMemsetAsync(S.nbc_d.p, 0, (size_t)ni * sizeof(int), S.stream), return false);
@@ -696,39 +776,62 @@ bool run_force(int nj, int ni, float eps2, bool nn, bool nbl) {
 }
 
 // Counts + lists back to the host; each list is sorted by j address (the reference's order,
-// gravity.c:888-900) and mapped to particle ids.  Lists longer than the capacity keep only
-// their count and set the overflow flag.
+// gravity.c:888-900) and mapped to particle ids on the device (g6_nb_sort_kernel).  Lists longer than
+// the capacity keep only their count and set the overflow flag.
 void nblist_collect(int ni) {
     S.nb_ni = ni;
     S.nb_error = 0;
     S.nbcounts.assign(ni, 0);
-    S.nblists.assign(ni, {});
-    // every list in j-address order, addresses replaced by ids, on the device
-    int P = 1;
-    while (P < nbmax()) P <<= 1;
-    if (ni > 0) {
-        g6_nb_sort_kernel<<<ni, 256, (size_t)P * sizeof(int), S.stream>>>(S.nbc_d.p, S.nbl_d.p, nbmax(), P, S.jd.p);
-        PGB_CUDA_OR(g_err, LIB, cudaGetLastError(), return);
-    }
-    if (S.nbc_h.reserve(ni) != cudaSuccess || S.nbl_h.reserve((size_t)ni * nbmax()) != cudaSuccess) {
-        raise(g_err, LIB, PGB_ERR_CUDA, "pinned neighbour-list buffer allocation failed");
-        return;
-    }
-    PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(S.nbc_h.p, S.nbc_d.p, (size_t)ni * sizeof(int), cudaMemcpyDeviceToHost,
-                                            S.stream), return);
-    PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(S.nbl_h.p, S.nbl_d.p, (size_t)ni * nbmax() * sizeof(int),
-                                            cudaMemcpyDeviceToHost, S.stream), return);
-    PGB_CUDA_OR(g_err, LIB, cudaStreamSynchronize(S.stream), return);
-    for (int i = 0; i < ni; i++) {
-        int c = S.nbc_h.p[i];
-        S.nbcounts[i] = c;
-        if (c > nbmax()) {
-            S.nb_error = 1;
-            continue;
+    const int cap = nbmax();
+    S.nbids.clear();
+    S.nboff.assign(ni, 0);
+    auto add_list = [](int i, int count, int stored) {
+        S.nbcounts[i] = count;
+        S.nboff[i] = S.nbids.size();
+        S.nbids.resize(S.nbids.size() + stored);
+        return S.nbids.data() + S.nboff[i];
+    };
+    if (S.wait_words) {
+        int i = 0, k = 0, c = -1;   // row, entry, entries (-1: not known yet)
+        int* list = nullptr;
+        const bool ok = take_words([&] {
+            for (; i < ni; i++, c = -1) {
+                const uint2* row = S.nbw.p + (size_t)i * (cap + 1);
+                if (c < 0) {
+                    int count;
+                    if (!take_word(row, S.seq, count)) return false;
+                    c = count > cap ? 0 : count;
+                    list = add_list(i, count, c);
+                    k = 0;
+                }
+                while (k < c && take_word(row + 1 + k, S.seq, list[k])) k++;
+                if (k < c) return false;
+            }
+            return true;
+        });
+        if (!ok) S.nbcounts.assign(ni, 0);
+    } else {
+        if (ni > 0) {
+            g6_nb_sort_kernel<<<ni, 256, nb_sort_smem(), S.stream>>>(S.nbc_d.p, S.nbl_d.p, cap, S.jd.p, nullptr, 0);
+            PGB_CUDA_OR(g_err, LIB, cudaGetLastError(), return);
         }
-        // sorted by j address and mapped to ids on the device (g6_nb_sort_kernel)
-        S.nblists[i].assign(S.nbl_h.p + (size_t)i * nbmax(), S.nbl_h.p + (size_t)i * nbmax() + c);
+        if (S.nbc_h.reserve(ni) != cudaSuccess || S.nbl_h.reserve((size_t)ni * cap) != cudaSuccess) {
+            raise(g_err, LIB, PGB_ERR_CUDA, "pinned neighbour-list buffer allocation failed");
+            return;
+        }
+        PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(S.nbc_h.p, S.nbc_d.p, (size_t)ni * sizeof(int), cudaMemcpyDeviceToHost,
+                                                S.stream), return);
+        PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(S.nbl_h.p, S.nbl_d.p, (size_t)ni * cap * sizeof(int),
+                                                cudaMemcpyDeviceToHost, S.stream), return);
+        PGB_CUDA_OR(g_err, LIB, cudaStreamSynchronize(S.stream), return);
+        for (int i = 0; i < ni; i++) {
+            const int count = S.nbc_h.p[i], c = count > cap ? 0 : count;
+            int* list = add_list(i, count, c);
+            if (c > 0) std::memcpy(list, S.nbl_h.p + (size_t)i * cap, (size_t)c * sizeof(int));
+        }
     }
+    for (int i = 0; i < ni; i++)
+        if (S.nbcounts[i] > cap) S.nb_error = 1;
 }
 
 // The common body of every g6calc_lasthalf* variant.
@@ -767,11 +870,12 @@ int lasthalf_impl(int nj, int ni, const int* pidx, const double (*pos)[3], const
     }
     bool nn = (nnb != nullptr);
     // eps2 is a per-call scalar, used as float (phantom_g6.c:191)
-    S.wait_flags = 0;
+    S.wait_words = false;
     if (!time_mark(0)) return 0;
     if (!run_force(nj, ni, (float)eps2, nn, nbl)) return 0;
     if (!time_mark(1)) return 0;
-    if (!wait_results() || !time_add()) return 0;
+    if (!wait_results(ni) || !time_add()) return 0;
+    S.uploading = false;   // the upload came before the results
     for (int i = 0; i < ni; i++) {
         const G6Out& o = S.outh.p[i];
         acc[i][0] = o.ax;
@@ -809,11 +913,11 @@ PGB_EXPORT void g6_close(int gpid) {
     S.st.release();
     S.pcnt.release();
     S.spart.release();
-    S.wait_flags = 0;
+    S.wait_words = false;
+    S.nbc_zero = false;
     S.nbc_d.release();
     S.nbl_d.release();
-    S.sbuf_d.release();
-    S.sidx_d.release();
+    S.uploading = false;
     for (int a : S.dirty) S.dirty_flag[a] = 0;
     S.dirty.clear();
     S.all_dirty = true;
@@ -837,7 +941,7 @@ PGB_EXPORT void g6_set_j_particle(int gpid, int padr, int pidx, double t, double
         return;
     }
     std::lock_guard<std::mutex> g(S.mu);
-    if (!grow_j(padr + 1)) return;
+    if (!grow_j(padr + 1) || !wait_upload()) return;
     G6Ptcl& p = S.jh.p[padr];
     for (int d = 0; d < 3; d++) {
         p.pos[d] = pos[d];
@@ -912,9 +1016,8 @@ PGB_EXPORT int g6_get_neighbour_list(int gpid, int ipipe, int maxlen, int* nblen
         return 1;
     }
     if (S.nbcounts[ipipe] > maxlen || S.nbcounts[ipipe] > nbmax()) return 1;
-    const std::vector<int>& v = S.nblists[ipipe];
-    *nblen = (int)v.size();
-    for (size_t k = 0; k < v.size(); k++) nbl[k] = v[k];
+    *nblen = S.nbcounts[ipipe];
+    if (*nblen > 0) std::memcpy(nbl, S.nbids.data() + S.nboff[ipipe], (size_t)*nblen * sizeof(int));
     return 0;
 }
 

@@ -133,11 +133,7 @@ __device__ __forceinline__ Group regular_group(const G6Args& A, int g) {
 
 // FP64 predictor: one thread per j (gravity.c:149-193; velocity stored as float, :168-173).
 // ff: store the predicted position in the double-float layout.
-__global__ void g6_predict_kernel(const G6Ptcl* __restrict__ p, int nj, double ti, G6PredJ* __restrict__ out,
-                                  bool ff) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nj) return;
-    const G6Ptcl& P = p[j];
+__device__ __forceinline__ G6PredJ g6_predict(const G6Ptcl& P, double ti, bool ff) {
     double dt = ti - P.tim;
     double dt2 = dt * dt, dt3 = dt2 * dt;
     G6PredJ o;
@@ -150,29 +146,86 @@ __global__ void g6_predict_kernel(const G6Ptcl* __restrict__ p, int nj, double t
     o.m = (float)P.mass;
     o.id = P.idx;
     o.pad = 0.f;
-    out[j] = o;
+    return o;
+}
+__global__ void g6_predict_kernel(const G6Ptcl* __restrict__ p, int nj, double ti, G6PredJ* __restrict__ out,
+                                  bool ff) {
+    int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < nj) out[j] = g6_predict(p[j], ti, ff);
 }
 
-// Sparse j-memory update: jd[idx[k]] = rec[k] (addresses checked against the capacity).
-__global__ void g6_scatter_kernel(const G6Ptcl* __restrict__ rec, const int* __restrict__ idx, int n, int cap,
-                                  G6Ptcl* __restrict__ jd) {
+// A 128-byte j record from mapped host memory, not through a cache that may hold an older one.
+__device__ __forceinline__ G6Ptcl g6_host_record(const G6Ptcl* rec) {
+    static_assert(sizeof(G6Ptcl) % 16 == 0, "whole 16-byte words");
+    G6Ptcl P;
+    uint4* d = reinterpret_cast<uint4*>(&P);
+#pragma unroll
+    for (int w = 0; w < (int)(sizeof(G6Ptcl) / 16); w++) d[w] = __ldcv(reinterpret_cast<const uint4*>(rec) + w);
+    return P;
+}
+
+// Sparse j-memory update: jd[idx[k]] = rec[k], both read from mapped host memory (addresses checked
+// against the capacity).
+__global__ void g6_scatter_kernel(const G6Ptcl* rec, const int* idx, int n, int cap, G6Ptcl* __restrict__ jd) {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    int a = idx[k];
-    if (a >= 0 && a < cap) jd[a] = rec[k];
+    int a = __ldcv(idx + k);
+    if (a >= 0 && a < cap) jd[a] = g6_host_record(rec + k);
+}
+
+// The same with the prediction of every j in one launch, for at most G6_UPD_MAX changed records,
+// whose addresses come in the parameter block: each CTA marks those of its own j range, and the
+// thread of a marked j takes the record from the host.
+constexpr int G6_UPD_MAX = 64;
+struct G6Update {
+    const G6Ptcl* rec;   // mapped host memory
+    int n;
+    int idx[G6_UPD_MAX];
+};
+__global__ void __launch_bounds__(256) g6_update_predict_kernel(G6Ptcl* jd, int cap,
+                                                                const __grid_constant__ G6Update U, int nj, double ti,
+                                                                G6PredJ* __restrict__ out, bool ff) {
+    __shared__ short s_src[256];
+    const int j0 = blockIdx.x * 256, j = j0 + (int)threadIdx.x;
+    s_src[threadIdx.x] = -1;
+    __syncthreads();
+    if (threadIdx.x < U.n) {
+        const int k = threadIdx.x;
+        const int l = U.idx[k] - j0;
+        if (l >= 0 && l < 256) s_src[l] = (short)k;
+    }
+    __syncthreads();
+    const int src = s_src[threadIdx.x];
+    if (j >= (src >= 0 ? cap : nj)) return;
+    const G6Ptcl P = src >= 0 ? g6_host_record(U.rec + src) : jd[j];
+    if (src >= 0) jd[j] = P;
+    if (j < nj) out[j] = g6_predict(P, ti, ff);
 }
 
 // Neighbour lists after the force launch: each i's entries were appended by atomics in
 // arrival order; this kernel (one CTA per i) sorts a list of count <= nbmax entries by j address
-// in shared memory (bitonic network over P >= count slots, P a power of two) and replaces every
+// in shared memory (bitonic network over the power of two >= count: 24 us for 33 lists of some tens of
+// entries when it ran over nbmax = 1024 slots) and replaces every
 // address by the id stored in the j-memory, so that the list is the reference's (j-address
 // order, gravity.c:888-900, ids).  A list longer than nbmax kept only its count and is left
 // alone (the host reports the overflow).
-__global__ void g6_nb_sort_kernel(const int* __restrict__ nb_count, int* __restrict__ nb_list, int nbmax, int P,
-                                  const G6Ptcl* __restrict__ jmem) {
+// host != nullptr: row i of the result goes to mapped host memory instead, nbmax + 1 words of
+// (value, seq), first the count and then the ids, and the count is zeroed for the next call.
+__global__ void g6_nb_sort_kernel(int* nb_count, int* __restrict__ nb_list, int nbmax,
+                                  const G6Ptcl* __restrict__ jmem, uint2* host, unsigned seq) {
     extern __shared__ int sh_nb[];
     const int c = nb_count[blockIdx.x];
+    uint2* out = host ? host + (size_t)blockIdx.x * (nbmax + 1) : nullptr;
+    if (out) {
+        __syncthreads();   // every thread has read the count
+        if (threadIdx.x == 0) {
+            nb_count[blockIdx.x] = 0;
+            __stwt(out, make_uint2((unsigned)c, seq));
+        }
+    }
     if (c > nbmax || c <= 0) return;
+    int P = 1;
+    while (P < c) P <<= 1;
     int* row = nb_list + (size_t)blockIdx.x * nbmax;
     for (int k = threadIdx.x; k < P; k += blockDim.x) sh_nb[k] = k < c ? row[k] : 0x7fffffff;
     __syncthreads();
@@ -191,7 +244,11 @@ __global__ void g6_nb_sort_kernel(const int* __restrict__ nb_count, int* __restr
             }
             __syncthreads();
         }
-    for (int k = threadIdx.x; k < c; k += blockDim.x) row[k] = jmem[sh_nb[k]].idx;
+    for (int k = threadIdx.x; k < c; k += blockDim.x) {
+        const int id = jmem[sh_nb[k]].idx;
+        if (out) __stwt(out + 1 + k, make_uint2((unsigned)id, seq));
+        else row[k] = id;
+    }
 }
 
 // FP32 partial sums cover at most G6_FOLD terms (per thread and i) before they are added into
@@ -618,17 +675,20 @@ __device__ __forceinline__ double2 word_finish(double2 v, bool w3) {
 // [wbeg, wbeg + nw) of a row (4 words per G6Out): thread (g, f) of R <= NT/nw row groups sums word
 // f of rows g, g+R, ... (coalesced 16-byte loads through L2, up to eight rows in flight), then
 // the R group sums are added in group order through shared memory W (NT words).  The order is
-// fixed for a given (NT, nw, nrows): deterministic.  finish: write the final scaled result (acc,
-// jerk x -1/8, pot x 1/2) instead of the raw sum.  dst (same word indexing) may be row 0 itself:
-// every word is read before it is written.
-template <int NT>
+// fixed for a given (NT, nw, nrows): deterministic.  store(f, v) takes the sum of word f -- the
+// final scaled result (acc, jerk x -1/8, pot x 1/2) with finish, else the raw sum -- and may write
+// row 0 itself: every word is read before it is written.
+struct G6StoreWords {
+    G6Out* dst;
+    __device__ __forceinline__ void operator()(int f, double2 v) const { reinterpret_cast<double2*>(dst)[f] = v; }
+};
+template <int NT, class Store>
 __device__ __forceinline__ void reduce_rows(const G6Out* base, size_t stride, int nrows, int wbeg, int nw,
-                                            G6Out* dst, bool finish, double2* W) {
+                                            Store store, bool finish, double2* W) {
     // row groups: as many as the threads allow, but no more than the rows and at most 8 (their
     // sums are combined serially)
     const int R = (2 * nw <= NT) ? min(min(NT / nw, nrows), 8) : 1;
     const double2* src = reinterpret_cast<const double2*>(base);
-    double2* out = reinterpret_cast<double2*>(dst);
     const size_t wstride = 4 * stride;
     for (int k0 = 0; k0 < nw; k0 += (R > 1 ? nw : NT)) {
         const int g = (R > 1) ? threadIdx.x / nw : 0;
@@ -675,7 +735,7 @@ __device__ __forceinline__ void reduce_rows(const G6Out* base, size_t stride, in
             continue;
         }
         if (finish) s0 = word_finish(s0, w3);
-        out[f] = s0;
+        store(f, s0);
     }
 }
 
@@ -1108,13 +1168,13 @@ __global__ void __launch_bounds__(NT, g6_min_ctas<NT, IPT, g6_uses_jp<IPT, FF, N
             const int nbk = min(B, G.nchunk - b * B);
             if (!group_arrive(A.bundle_counters, r0, nbk, &s_flag)) continue;
             G6Out* row0 = A.partial + (size_t)r0 * A.itile;
-            reduce_rows<NT>(row0, (size_t)A.itile, nbk, 0, 4 * G.ni, row0, false, W);
+            reduce_rows<NT>(row0, (size_t)A.itile, nbk, 0, 4 * G.ni, G6StoreWords{row0}, false, W);
             const int nb = (G.nchunk + B - 1) / B;
             if (!group_arrive(A.group_counters, T.group, nb, &s_flag)) continue;
-            reduce_rows<NT>(A.partial + (size_t)G.slot0 * A.itile, (size_t)B * A.itile, nb, 0, 4 * G.ni, out, true, W);
+            reduce_rows<NT>(A.partial + (size_t)G.slot0 * A.itile, (size_t)B * A.itile, nb, 0, 4 * G.ni, G6StoreWords{out}, true, W);
         } else {
             if (!group_arrive(A.group_counters, T.group, G.nchunk, &s_flag)) continue;
-            reduce_rows<NT>(A.partial + (size_t)G.slot0 * A.itile, (size_t)A.itile, G.nchunk, 0, 4 * G.ni, out, true, W);
+            reduce_rows<NT>(A.partial + (size_t)G.slot0 * A.itile, (size_t)A.itile, G.nchunk, 0, 4 * G.ni, G6StoreWords{out}, true, W);
         }
         if constexpr (NN && g6_quad_min<IPT, FF, NBL, JP>()) {
             __syncthreads();

@@ -5,18 +5,24 @@
 // Such a call has far too few i-particles to fill the GPU by i, so the j-range is cut into one
 // chunk per CTA (gridDim.x chunks, every CTA resident) and the partial sums are reduced in
 // three fixed-order stages, none of which round-trips through a task scheduler:
-//   1. the JL j-lanes of the CTA, word by word through shared memory (lane order);
+//   1. the JL j-lanes of the CTA, word by word through shared memory: groups of lanes in lane
+//      order, then the groups (all lanes one after another took 2.5 us of a 7 x 1024 call, this
+//      0.8);
 //   2. the CTAs of a thread-block cluster (CL consecutive chunks), through distributed shared
 //      memory: CTA `rank` sums its slice of the words over the cluster's CTAs (rank order) and
 //      writes the cluster's row of partial sums;
 //   3. the cluster rows: slice r of the words of every row is written by rank r of each
 //      cluster, and the rank-r CTA that arrives last on a per-slice counter sums the slice over
 //      the rows (reduce_rows: fixed row order) and writes the final scaled result -- CL CTAs
-//      share the final stage and no cluster waits for another.
+//      share the final stage and no cluster waits for another.  A call of one cluster ends with
+//      stage 2.
 // The i-records come in the parameter block (no upload; staged to shared memory with
 // broadcast reads) and the j-chunks are a pure function of (blockIdx, nj, gridDim), so a call
 // is one launch.  The result is deterministic for a given
 // grid and cluster size.  Per pair the arithmetic is g6_pair(), identical to g6_kernel.
+// The results go to the host as numbered words (G6HostWords).  Latency bounds the kernel: 4 us for
+// 7 x 1024 (1.2 to the last pair), 14 us for 48 x 65536 (7.3 to the last pair, 3 in the clusters, 2.5 in
+// the last stage), before 14 and 22 us to the flag behind the results' fence.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -31,37 +37,41 @@ struct G6SmallArgs {
     int ni, nj;        // i-particles (<= ISL) and j-records [0, nj)
     G6Out* partial;    // [gridDim.x / CL][ISL] cluster sums
     int* counter;      // [cluster size] arrivals per word slice; zero at launch, reset by the last
-    G6Out* out;        // [ni] final results
     int* nb_count;     // neighbour lists (NBL), indexed by i
     int* nb_list;
     int nb_maxlen;
-    // completion flags in mapped host memory (nullptr: none): the CTA that writes word slice r
-    // of the results sets done[r] = seq after them, so the host can wait for the results by
-    // polling instead of synchronising the stream
-    volatile unsigned* done;
+    // final results in mapped host memory: result word f (16 bytes, 4 to a G6Out) as words[2f],
+    // words[2f + 1], each two 32-bit values with the call's number after each
+    uint4* words;
     unsigned seq;
 };
 
-// Publish a final slice: every thread's result writes are made visible to the host before
-// thread 0 sets the slice's completion flag.
-__device__ __forceinline__ void publish_done(const G6SmallArgs& A, int slice) {
-    if (!A.done) return;
-    __threadfence_system();
-    __syncthreads();
-    if (threadIdx.x == 0) A.done[slice] = A.seq;
-}
+// A result word for the host.  Every 8 bytes carry the call's number themselves, so the host takes a
+// word as soon as it is there and no store waits for another: with plain words, a system fence and a
+// flag after it the fence alone took 6.3 us of the 14 us of a call of 7 i against 1024 j.
+struct G6HostWords {
+    uint4* words;
+    unsigned seq;
+    __device__ __forceinline__ void operator()(int f, double2 v) const {
+        const unsigned long long x = __double_as_longlong(v.x), y = __double_as_longlong(v.y);
+        __stwt(words + 2 * f, make_uint4((unsigned)x, seq, (unsigned)(x >> 32), seq));
+        __stwt(words + 2 * f + 1, make_uint4((unsigned)y, seq, (unsigned)(y >> 32), seq));
+    }
+};
 
 constexpr int G6_SMALL_MAXI = 64;
+constexpr int SMALL_CL_MAX = 8;   // CTAs per cluster at most (the portable limit)
 
 // The i-records of a small call, passed by value in the kernel's parameter block: no separate
 // upload (and no host-to-device copy latency) for a call of up to G6_SMALL_MAXI i-particles.
+template <int ISL>
 struct G6IBlock {
-    G6I rec[G6_SMALL_MAXI];
+    G6I rec[ISL];
 };
 
 template <int ISL, int JL, bool FF, bool NN, bool NBL>
 __global__ void __launch_bounds__(ISL * JL, 2)
-    g6_small_kernel(const G6SmallArgs A, const __grid_constant__ G6IBlock ib) {
+    g6_small_kernel(const G6SmallArgs A, const __grid_constant__ G6IBlock<ISL> ib) {
     namespace cg = cooperative_groups;
     constexpr int NT = ISL * JL;
     static_assert(ISL <= G6_SMALL_MAXI, "i-slots within the i-block");
@@ -124,66 +134,83 @@ __global__ void __launch_bounds__(ISL * JL, 2)
         __syncthreads();
     }
 
-    // 1. j-lanes: thread w = 4 slot + word sums that word over the lanes in order
-    __syncthreads();
-    {
-        G6Out o;
-        o.ax = S[0]; o.ay = S[1]; o.az = S[2];
-        o.jx = S[3]; o.jy = S[4]; o.jz = S[5];
-        o.pot = S[6];
-        o.key = kmin;
-        o.jadr = kadr;
-        reinterpret_cast<G6Out*>(smem)[threadIdx.x] = o;
-    }
-    __syncthreads();
+    // 1. j-lanes, word by word: thread (g, wd, s) sums word wd of slot s over its NT / (4 ISL)-th of
+    //    the lanes in order, then the parts are added in order
+    constexpr int NW = 4 * ISL, NG = NT / NW, PER = (JL + NG - 1) / NG;
+    double2* sw = reinterpret_cast<double2*>(smem);   // [4][NT], word by word: no bank conflicts
+    const G6HostWords host{A.words, A.seq};
     const int nw = 4 * A.ni;
-    const double2* rw = reinterpret_cast<const double2*>(smem);
-    if (threadIdx.x < nw) {
-        const bool w3 = (threadIdx.x & 3) == 3;
-        const int s = threadIdx.x >> 2, wd = threadIdx.x & 3;
-        double2 v = rw[4 * s + wd];
-        for (int l = 1; l < JL; l++) v = word_add(v, rw[4 * (l * ISL + s) + wd], w3);
-        if (nch == 1) {
-            // the whole call in one CTA: final result directly
-            reinterpret_cast<double2*>(A.out)[threadIdx.x] = word_finish(v, w3);
-        }
-        cta_w[threadIdx.x] = v;
+    const int wd = (int)threadIdx.x / ISL % 4, g = (int)threadIdx.x / NW;
+    __syncthreads();
+    sw[threadIdx.x] = make_double2(S[0], S[1]);
+    sw[NT + threadIdx.x] = make_double2(S[2], S[3]);
+    sw[2 * NT + threadIdx.x] = make_double2(S[4], S[5]);
+    sw[3 * NT + threadIdx.x] = make_double2(
+        S[6], __longlong_as_double((long long)((unsigned long long)(unsigned)kadr << 32 |
+                                               (unsigned)__float_as_int(kmin))));
+    __syncthreads();
+    const bool mine = g < NG && slot < A.ni, w3 = wd == 3;
+    double2 v = word_zero(w3);
+    if (mine) {
+        const double2* col = sw + wd * NT + slot;
+        double2 u[PER];
+#pragma unroll
+        for (int k = 0; k < PER; k++)
+            if (g * PER + k < JL) u[k] = col[(g * PER + k) * ISL];
+        v = u[0];
+#pragma unroll
+        for (int k = 1; k < PER; k++)
+            if (g * PER + k < JL) v = word_add(v, u[k], w3);
     }
-    if (nch == 1) {
-        publish_done(A, 0);
-        return;
+    __syncthreads();
+    if (mine && g > 0) sw[threadIdx.x] = v;
+    __syncthreads();
+    if (mine && g == 0) {
+#pragma unroll
+        for (int k = 1; k < NG; k++) v = word_add(v, sw[k * NW + threadIdx.x], w3);
+        const int f = 4 * slot + wd;
+        if (nch == 1) host(f, word_finish(v, w3));   // the whole call in one CTA
+        cta_w[f] = v;
     }
+    if (nch == 1) return;
 
     // 2. the cluster: CTA `rank` reduces words [f0, f1) over the cluster's CTAs, in rank order,
-    //    into the cluster's row
+    //    into the cluster's row (the only cluster: into the result)
     cg::cluster_group cl = cg::this_cluster();
     const int CL = (int)cl.num_blocks(), rank = (int)cl.block_rank();
     cl.sync();
+    const int nclus = nch / CL;
     const int f0 = rank * nw / CL, f1 = (rank + 1) * nw / CL;
     const int f = f0 + (int)threadIdx.x;
     if (f < f1) {
-        const bool w3 = (f & 3) == 3;
-        double2 v = *cl.map_shared_rank(&cta_w[f], 0);
-        for (int q = 1; q < CL; q++) v = word_add(v, *cl.map_shared_rank(&cta_w[f], q), w3);
-        reinterpret_cast<double2*>(A.partial + (size_t)(c / CL) * ISL)[f] = v;
+        const bool fw3 = (f & 3) == 3;
+        double2 q[SMALL_CL_MAX];
+#pragma unroll
+        for (int k = 0; k < SMALL_CL_MAX; k++)
+            if (k < CL) q[k] = *cl.map_shared_rank(&cta_w[f], k);
+        double2 t = q[0];
+#pragma unroll
+        for (int k = 1; k < SMALL_CL_MAX; k++)
+            if (k < CL) t = word_add(t, q[k], fw3);
+        if (nclus == 1) host(f, word_finish(t, fw3));
+        else reinterpret_cast<double2*>(A.partial + (size_t)(c / CL) * ISL)[f] = t;
     }
 
     // 3. slice `rank` of every cluster row was written by that cluster's CTA `rank`: those CTAs
     //    arrive on counter[rank], and the last of them sums the slice over the rows in order
-    const int nclus = nch / CL;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int prev = atomicAdd(&A.counter[rank], 1);
-        const int last = (prev == nclus - 1);
-        if (last) atomicExch(&A.counter[rank], 0);
-        s_flag = last;
-    }
-    __syncthreads();
-    if (s_flag) {
-        __threadfence();
-        reduce_rows<NT>(A.partial, (size_t)ISL, nclus, f0, f1 - f0, A.out, true, reinterpret_cast<double2*>(smem));
-        publish_done(A, rank);
+    if (nclus > 1) {
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            __threadfence();
+            const int prev = atomicAdd(&A.counter[rank], 1);
+            const int last = (prev == nclus - 1);
+            if (last) atomicExch(&A.counter[rank], 0);
+            __threadfence();
+            s_flag = last;
+        }
+        __syncthreads();
+        if (s_flag)
+            reduce_rows<NT>(A.partial, (size_t)ISL, nclus, f0, f1 - f0, host, true, reinterpret_cast<double2*>(smem));
     }
     cl.sync();  // no CTA leaves while a peer may still read its cta_w
 }
