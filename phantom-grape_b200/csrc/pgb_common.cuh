@@ -265,11 +265,20 @@ struct Stager {
     DevBuf<ORec> dpart;            // partial rows, [rows][itile]
     HostBuf<unsigned char> hcall;  // pinned staging of the call block
     cudaEvent_t copied = nullptr;  // last H2D copy out of hcall
-    size_t off_g = 0, off_i = 0, off_bc = 0;
+    size_t off_g = 0, off_i = 0, off_bc = 0, total = 0;
     int ntasks = 0;
 
     cudaError_t stage(cudaStream_t s, const std::vector<Task>& tasks, const std::vector<Group>& groups, int rows,
                       int itile, const IRec* i_host, int ni_host, size_t min_groups = 0) {
+        cudaError_t e = prepare(s, tasks, groups, rows, itile, ni_host, min_groups);
+        if (e != cudaSuccess) return e;
+        if (ni_host) std::memcpy(irecs_host(), i_host, (size_t)ni_host * sizeof(IRec));
+        return upload(s);
+    }
+    // The call block in hcall but for the i-records, which the caller writes to irecs_host(); then
+    // upload().
+    cudaError_t prepare(cudaStream_t s, const std::vector<Task>& tasks, const std::vector<Group>& groups, int rows,
+                        int itile, int ni_host, size_t min_groups = 0) {
         cudaError_t e;
         if (!copied && (e = cudaEventCreateWithFlags(&copied, cudaEventDisableTiming)) != cudaSuccess) return e;
         // the previous copy out of hcall must have left before hcall is rewritten
@@ -277,19 +286,20 @@ struct Stager {
         const size_t off_t = 16;
         off_g = (off_t + tasks.size() * sizeof(Task) + 15) & ~size_t(15);
         off_i = (off_g + groups.size() * sizeof(Group) + 15) & ~size_t(15);
-        size_t total = off_i + (size_t)ni_host * sizeof(IRec);
+        total = off_i + (size_t)ni_host * sizeof(IRec);
         if ((e = hcall.reserve(total)) != cudaSuccess) return e;
         if ((e = dcall.reserve(total)) != cudaSuccess) return e;
         std::memset(hcall.p, 0, 16);
         if (!tasks.empty()) std::memcpy(hcall.p + off_t, tasks.data(), tasks.size() * sizeof(Task));
         if (!groups.empty()) std::memcpy(hcall.p + off_g, groups.data(), groups.size() * sizeof(Group));
-        if (ni_host) std::memcpy(hcall.p + off_i, i_host, (size_t)ni_host * sizeof(IRec));
-        if ((e = reserve_scratch(s, rows, itile, std::max(groups.size(), min_groups))) != cudaSuccess) return e;
-        if ((e = cudaMemcpyAsync(dcall.p, hcall.p, total, cudaMemcpyHostToDevice, s)) != cudaSuccess) return e;
-        if ((e = cudaEventRecord(copied, s)) != cudaSuccess) return e;
         ntasks = (int)tasks.size();
-        return cudaSuccess;
+        return reserve_scratch(s, rows, itile, std::max(groups.size(), min_groups));
     }
+    cudaError_t upload(cudaStream_t s) {
+        const cudaError_t e = cudaMemcpyAsync(dcall.p, hcall.p, total, cudaMemcpyHostToDevice, s);
+        return e != cudaSuccess ? e : cudaEventRecord(copied, s);
+    }
+    IRec* irecs_host() { return (IRec*)(hcall.p + off_i); }
     // Partial rows and zeroed counters: one per group (`ngroups` includes groups that the
     // kernel derives itself, regular mode), then one per partial row for the two-level
     // reduction of long groups.  Enough for a launch that uploads nothing.

@@ -25,6 +25,8 @@
 //    phantom_g5.c:148-166 read one record past the end).
 //  * j-memory capacity is 1 Mi records (PGB_G5_JMEMSIZE), not 64 Ki; exceeding it is an error,
 //    not an out-of-bounds write.
+#include <chrono>
+
 #include "pgb_g5_kernels.cuh"
 
 using namespace pgb;
@@ -333,18 +335,19 @@ inline float scale_i(double x) {
 struct Launcher {
     Stager<float4, double4> st;
 
-    bool stage(cudaStream_t s, const std::vector<Task>& tasks, const std::vector<Group>& groups, int rows, int itile,
-               const float4* i_host, int ni_host) {
-        PGB_CUDA_OR(g_err, LIB, st.stage(s, tasks, groups, rows, itile, i_host, ni_host), return false);
+    bool stage(cudaStream_t s, const std::vector<Task>& tasks, const std::vector<Group>& groups, int rows, int itile) {
+        PGB_CUDA_OR(g_err, LIB, st.stage(s, tasks, groups, rows, itile, nullptr, 0), return false);
         return true;
     }
 
     // Launch over the staged work list.  The kernel leaves its task counter at zero, so the same
     // staged list can be launched again (e.g. from a CUDA graph) without a reset.
     bool launch(int kind, int cfg, cudaStream_t s, const float4* i_dev, const float4* jpos, const float4* jaux,
-                double4* out, const int* jidx = nullptr) {
+                double4* out, const int* jidx = nullptr, uint4* words = nullptr, unsigned seq = 0) {
         if (st.ntasks <= 0) return true;
         G5Args a;
+        a.words = words;
+        a.seq = seq;
         a.ipos = i_dev ? i_dev : st.irecs();
         a.jpos = jpos;
         a.jaux = jaux;
@@ -366,6 +369,7 @@ struct Launcher {
         int slots = sm_count(g_device) * occupancy_of(kind, cfg);
         int grid = st.ntasks < slots ? st.ntasks : slots;
         PGB_CUDA_OR(g_err, LIB, launch_kind(kind, cfg, grid, a, s), return false);
+        if (!i_dev) return true;   // a call's own list: the call waits for its results
         // completion marker for pgb5_plan_update; a launch captured into a CUDA graph records
         // none (its replays are the caller's to finish before the plan is updated)
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -409,7 +413,8 @@ struct Dev {
     float4 ip[MAXPIPE];
     DevBuf<double4> outd;
     HostBuf<double4> outh;
-    HostBuf<float4> ibuf;
+    HostBuf<uint2> words;   // results of a call that sends words, [ni][8] of (value, call number)
+    unsigned seq = 0;       // number of the last such call
     int pending = 0;     // number of results of the last g5_run / g5c_run (0: none)
     bool inflight = false;  // a g5_run has not been synchronised yet
     Launcher L;
@@ -511,17 +516,37 @@ bool flush_c(Dev& d) {
     return true;
 }
 
-// Launch `kind` for ni i-records (host) against this devid's j-memory (nbody records) or cell
-// memory (ncell cells).  Results land in d.outh after the stream synchronises.
-bool compute(Dev& d, int kind, int ni, const float4* ih) {
+// A call of at most this many i sends its results as words that the host takes as they arrive; a larger
+// one copies them (half the bytes) and waits for the stream.  Measured (us a call, copied / words): 250 x 250
+// 52 / 40, 999 x 999 53 / 48, 2000 63 / 58, 4096 99 / 87.
+constexpr int G5_WORDS_NI = 4096;
+bool sends_words(int kind, int ni) { return ni <= G5_WORDS_NI && G5C_NT[pick_cfg(kind, ni)] == G5S_NT; }
+
+// Launch `kind` for ni i-records, which fill(dst) writes, against this devid's j-memory (nbody records)
+// or cell memory (ncell cells).  The results land in d.outh after the stream synchronises, or, with
+// `words`, in d.words (numbered d.seq).
+template <class Fill>
+bool compute(Dev& d, int kind, int ni, Fill fill, bool words) {
     int nj = kind == G5_QUAD ? d.ncell : d.nbody;
+    // the j-records go out while the i-records are converted (straight into the call block: 16384 x 16384
+    // 290 -> 281 us)
     if (kind == G5_QUAD) {
         if (!grow_c(d, nj > 0 ? nj : 1) || !flush_c(d)) return false;
     } else {
         if (!grow_j(d, nj > 0 ? nj : 1) || !flush_j(d)) return false;
     }
-    PGB_CUDA_OR(g_err, LIB, d.outd.reserve(ni > 0 ? ni : 1), return false);
-    PGB_CUDA_OR(g_err, LIB, d.outh.reserve(ni > 0 ? ni : 1), return false);
+    if (words) {
+        const size_t had = d.words.n;
+        PGB_CUDA_OR(g_err, LIB, d.words.reserve(8 * (size_t)ni, false, cudaHostAllocPortable | cudaHostAllocMapped),
+                    return false);
+        // no word carries the number of a call to come
+        const bool wrap = ++d.seq == 0;
+        if (wrap) d.seq = 1;
+        if (wrap || d.words.n != had) std::memset((void*)d.words.p, 0, d.words.n * sizeof(uint2));
+    } else {
+        PGB_CUDA_OR(g_err, LIB, d.outd.reserve(ni > 0 ? ni : 1), return false);
+        PGB_CUDA_OR(g_err, LIB, d.outh.reserve(ni > 0 ? ni : 1), return false);
+    }
     std::vector<Task> tasks;
     std::vector<Group> groups;
     const int cfg = pick_cfg(kind, ni);
@@ -532,9 +557,13 @@ bool compute(Dev& d, int kind, int ni, const float4* ih) {
     int rows = plan_item(tasks, groups, 0, ni, 0, nj, itile, jchunk, 0);
     const float4* jpos = kind == G5_QUAD ? d.cd.p : d.jd.p;
     const float4* jaux = kind == G5_QUAD ? d.cqd.p : (kind == G5_SYMMETRIC ? d.jed.p : nullptr);
-    if (!d.L.stage(d.stream, tasks, groups, rows, itile, ih, ni)) return false;
-    if (!d.L.launch(kind, cfg, d.stream, nullptr, jpos, jaux, d.outd.p)) return false;
-    if (ni > 0)
+    auto& st = d.L.st;
+    PGB_CUDA_OR(g_err, LIB, st.prepare(d.stream, tasks, groups, rows, itile, ni), return false);
+    if (ni > 0) fill(st.irecs_host());
+    PGB_CUDA_OR(g_err, LIB, st.upload(d.stream), return false);
+    if (!d.L.launch(kind, cfg, d.stream, nullptr, jpos, jaux, d.outd.p, nullptr, words ? (uint4*)d.words.p : nullptr,
+                    d.seq)) return false;
+    if (ni > 0 && !words)
         PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(d.outh.p, d.outd.p, (size_t)ni * sizeof(double4),
                                                 cudaMemcpyDeviceToHost, d.stream), return false);
     return true;
@@ -546,17 +575,47 @@ bool sync_dev(Dev& d) {
     return true;
 }
 
-void write_out(const double4* o, int ni, double (*a)[3], double* p) {
-    for (int i = 0; i < ni; i++) {
-        a[i][0] = o[i].x;
-        a[i][1] = o[i].y;
-        a[i][2] = o[i].z;
+inline void write_one(const double (&o)[4], int i, double (*a)[3], double* p) {
+    a[i][0] = o[0];
+    a[i][1] = o[1];
+    a[i][2] = o[2];
 #ifdef PGB_TABLE
-        p[i] = 0.0;      // the table kernel computes no potential (PG5/table phantom_g5.c:145-154)
+    p[i] = 0.0;   // the table kernel computes no potential (PG5/table phantom_g5.c:145-154)
 #else
-        p[i] = -o[i].w;  // GRAPE-5 return sign (phantom_g5.c:251-259)
+    p[i] = -o[3];   // GRAPE-5 return sign (phantom_g5.c:251-259)
 #endif
+}
+void write_out(const double4* o, int ni, double (*a)[3], double* p) {
+    for (int i = 0; i < ni; i++) write_one({o[i].x, o[i].y, o[i].z, o[i].w}, i, a, p);
+}
+
+// The results of a call that sends words, as they arrive: a bounded spin, then the stream
+// synchronisation that reports a failed launch.
+bool take_words(Dev& d, int ni, double (*a)[3], double* p) {
+    const volatile unsigned long long* w = (const volatile unsigned long long*)d.words.p;
+    int i = 0;
+    auto take = [&] {
+        for (; i < ni; i++) {
+            double o[4];
+            for (int c = 0; c < 4; c++) {
+                const unsigned long long lo = w[8 * (size_t)i + 2 * c], hi = w[8 * (size_t)i + 2 * c + 1];
+                if ((unsigned)(lo >> 32) != d.seq || (unsigned)(hi >> 32) != d.seq) return false;
+                const unsigned long long v = hi << 32 | (lo & 0xffffffffull);
+                std::memcpy(&o[c], &v, sizeof v);
+            }
+            write_one(o, i, a, p);
+        }
+        return true;
+    };
+    auto t0 = std::chrono::steady_clock::now();
+    for (long it = 0;; it++) {
+        if (take()) return true;
+        if ((it & 1023) == 1023 && std::chrono::steady_clock::now() - t0 > std::chrono::seconds(5)) break;
     }
+    if (!sync_dev(d)) return false;
+    if (take()) return true;
+    raise(g_err, LIB, PGB_ERR_DEVICE, "a call's results did not arrive");
+    return false;
 }
 
 // The current xscale of the table library (building the default table on first use, as
@@ -604,7 +663,7 @@ void run_impl(int devid, int kind) {
     std::lock_guard<std::mutex> g(d->mu);
     int n = npipes();
     if (!quiesce(*d)) return;
-    if (compute(*d, kind, n, d->ip)) {
+    if (compute(*d, kind, n, [&](float4* r) { std::memcpy(r, d->ip, n * sizeof(float4)); }, false)) {
         d->pending = n;
         d->inflight = true;
     }
@@ -632,14 +691,17 @@ void calc_impl(int devid, int kind, const double (*x)[3], const double* eps2, do
     Dev* dj = d;
     std::lock_guard<std::mutex> g(dj->mu);
     if (!quiesce(*dj)) return;
-    if (dj->ibuf.reserve(ni) != cudaSuccess) {
-        raise(g_err, LIB, PGB_ERR_CUDA, "pinned i-buffer allocation failed (%d)", ni);
-        return;
+    const float e_all = (float)(g_eps * g_eps);
+    const bool words = sends_words(kind, ni);
+    auto fill = [&](float4* r) {
+        for (int i = 0; i < ni; i++) r[i] = make_i(x[i], eps2 ? (float)eps2[i] : e_all);
+    };
+    if (!compute(*dj, kind, ni, fill, words)) return;
+    if (words) {
+        take_words(*dj, ni, a, p);
+    } else if (sync_dev(*dj)) {
+        write_out(dj->outh.p, ni, a, p);
     }
-    float e_all = (float)(g_eps * g_eps);
-    for (int i = 0; i < ni; i++) dj->ibuf.p[i] = make_i(x[i], eps2 ? (float)eps2[i] : e_all);
-    if (!compute(*dj, kind, ni, dj->ibuf.p) || !sync_dev(*dj)) return;
-    write_out(dj->outh.p, ni, a, p);
 }
 
 }  // namespace
@@ -1083,7 +1145,7 @@ void set_tuned(long long key, int cfg) {
 }
 
 bool stage_plan(pgb5_plan* P, cudaStream_t s) {
-    return P->L.stage(s, P->tasks, P->groups, P->rows, cfg_itile(P->cfg), nullptr, 0);
+    return P->L.stage(s, P->tasks, P->groups, P->rows, cfg_itile(P->cfg));
 }
 }  // namespace
 

@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256) g6_update_predict_kernel(G6Ptcl* jd, int 
 
 // Neighbour lists after the force launch: each i's entries were appended by atomics in
 // arrival order; this kernel (one CTA per i) sorts a list of count <= nbmax entries by j address
-// in shared memory (bitonic network over the power of two >= count: 24 us for 33 lists of some tens of
+// in shared memory (bitonic network over the power of two >= count: 21 us for 33 lists of some tens of
 // entries when it ran over nbmax = 1024 slots) and replaces every
 // address by the id stored in the j-memory, so that the list is the reference's (j-address
 // order, gravity.c:888-900, ids).  A list longer than nbmax kept only its count and is left
