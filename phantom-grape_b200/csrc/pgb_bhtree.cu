@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(SC_NT) scan_partial(const T* in, long long n, 
 template <class T>
 __global__ void __launch_bounds__(SC_NT) scan_final(const T* in, long long n, const T* boff, T* out) {
     __shared__ T sh[SC_NT / 32];
+    if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = boff[gridDim.x];
     const long long b0 = (long long)blockIdx.x * SC_TILE + (long long)threadIdx.x * SC_PER;
     T v[SC_PER];
     T s = 0;
@@ -116,37 +117,54 @@ __global__ void __launch_bounds__(SC_NT) scan_final(const T* in, long long n, co
     }
 }
 
-// out[k] = sum_{j<k} in[j] for k <= n (out has n + 1 entries; in and out may not alias).
-// tmp: the block-sum buffers of the levels (two per level; the vector is sized once, before
-// any reference into it is taken, so the recursion never reallocates it).
-constexpr int SC_MAXLVL = 8;
+// A whole scan by one CTA, tile after tile.
 template <class T>
-bool excl_scan(const T* in, long long n, T* out, cudaStream_t s, std::vector<DevBuf<T>>& tmp, int lvl = 0) {
-    const long long nb = (n + SC_TILE - 1) / SC_TILE;
-    if (lvl == 0 && (int)tmp.size() < 2 * SC_MAXLVL) tmp.resize(2 * SC_MAXLVL);
-    if (lvl >= SC_MAXLVL) {
-        raise(g_err, LIB, PGB_ERR_CAPACITY, "prefix sum of %lld entries: too many levels", n);
-        return false;
+__global__ void __launch_bounds__(SC_NT) scan_one(const T* in, long long n, T* out) {
+    __shared__ T sh[SC_NT / 32];
+    T carry = 0;
+    for (long long t0 = 0; t0 < n; t0 += SC_TILE) {
+        const long long b0 = t0 + (long long)threadIdx.x * SC_PER;
+        T v[SC_PER];
+        T s = 0;
+#pragma unroll
+        for (int r = 0; r < SC_PER; r++) {
+            v[r] = (b0 + r < n) ? in[b0 + r] : T(0);
+            s += v[r];
+        }
+        T tot;
+        T run = carry + block_excl_scan<T>(s, sh, &tot);
+        carry += tot;
+#pragma unroll
+        for (int r = 0; r < SC_PER; r++) {
+            if (b0 + r < n) out[b0 + r] = run;
+            run += v[r];
+        }
     }
-    DevBuf<T>& bs = tmp[2 * lvl];
-    DevBuf<T>& bo = tmp[2 * lvl + 1];
-    PGB_CUDA_OR(g_err, LIB, bs.reserve((size_t)nb + 1), return false);
-    PGB_CUDA_OR(g_err, LIB, bo.reserve((size_t)nb + 2), return false);
+    if (threadIdx.x == 0) out[n] = carry;
+}
+
+// out[k] = sum_{j<k} in[j] for k <= n (out has n + 1 entries; in and out may not alias): one launch for a
+// tile, else three (block sums, their scan, the blocks).  A build makes some 40 scans, most of them of
+// a tile; with the block sums scanned by recursion and the totals copied, one of a tile took five
+// stream operations, a longer one eight.
+// tmp: the block sums and their scan.
+template <class T>
+bool excl_scan(const T* in, long long n, T* out, cudaStream_t s, std::vector<DevBuf<T>>& tmp) {
+    const long long nb = (n + SC_TILE - 1) / SC_TILE;
     if (n == 0) {
         PGB_CUDA_OR(g_err, LIB, cudaMemsetAsync(out, 0, sizeof(T), s), return false);
         return true;
     }
-    scan_partial<T><<<(unsigned)nb, SC_NT, 0, s>>>(in, n, bs.p);
     if (nb == 1) {
-        PGB_CUDA_OR(g_err, LIB, cudaMemsetAsync(bo.p, 0, sizeof(T), s), return false);
-        PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(bo.p + 1, bs.p, sizeof(T), cudaMemcpyDeviceToDevice, s),
-                    return false);
-    } else if (!excl_scan<T>(bs.p, nb, bo.p, s, tmp, lvl + 1)) {
-        return false;
+        scan_one<T><<<1, SC_NT, 0, s>>>(in, n, out);
+    } else {
+        if (tmp.size() < 2) tmp.resize(2);
+        PGB_CUDA_OR(g_err, LIB, tmp[0].reserve((size_t)nb), return false);
+        PGB_CUDA_OR(g_err, LIB, tmp[1].reserve((size_t)nb + 1), return false);
+        scan_partial<T><<<(unsigned)nb, SC_NT, 0, s>>>(in, n, tmp[0].p);
+        scan_one<T><<<1, SC_NT, 0, s>>>(tmp[0].p, nb, tmp[1].p);
+        scan_final<T><<<(unsigned)nb, SC_NT, 0, s>>>(in, n, tmp[1].p, out);
     }
-    scan_final<T><<<(unsigned)nb, SC_NT, 0, s>>>(in, n, bo.p, out);
-    // the total
-    PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(out + n, bo.p + nb, sizeof(T), cudaMemcpyDeviceToDevice, s), return false);
     PGB_CUDA_OR(g_err, LIB, cudaGetLastError(), return false);
     return true;
 }
@@ -636,17 +654,19 @@ __device__ __forceinline__ double box_d2(const double* p, const double g[3], dou
     return d2;
 }
 
-// The interaction lists are made by HT_UNITS work units per group, so that the walks spread
-// over many threads: unit u, whose base-8 digits (o_1 .. o_D, most significant first) name a
-// node D levels below the root, produces the part of the group's list that the host builder's
-// depth-first walk (make_interaction_list) produces inside that node's subtree.  Where the walk
-// takes a node of level l < D whole (its particle, itself as a cell, or its particles), the unit
-// whose digits below l are zero emits it.  The units' lists, concatenated in unit order, are the
-// group's list.  Most of a group's list lies in the few units around the group itself, so the
-// depth sets how many threads share that work: at D = 2 the long walks of an N = 2^20 tree fill
-// ~3 warps per SM.
-constexpr int HT_UNIT_LEVELS = 2;
-constexpr int HT_UNITS = 1 << (3 * HT_UNIT_LEVELS);
+// The interaction lists are made by 2^ulog work units per group, so that the walks spread
+// over many threads: unit u produces the part of the group's list that the host builder's
+// depth-first walk (make_interaction_list) takes from the nodes with pre-order numbers
+// [unit_begin(u), unit_begin(u + 1)).  The units' lists, concatenated in unit order, are the group's
+// list.  Cut by node numbers the units have equal shares of any tree: of a Hernquist sphere the units
+// of the 64 cells two levels below the root, which they replace, left nearly all particles to the
+// eight around the centre.
+struct Units {
+    int ulog, nn;
+    __device__ __forceinline__ int begin(int u) const { return (int)(((long long)u * nn) >> ulog); }
+    // the unit that holds node v (about)
+    __device__ __forceinline__ int of(int v) const { return (int)(((long long)v << ulog) / nn); }
+};
 // threads per block of the list walks: a block stays resident until its slowest walk ends, so
 // smaller blocks keep fewer finished warps idle (N = 2^22 build: 12.3 ms with 128, 12.7 with
 // 64, 13.0 with 256 threads)
@@ -654,11 +674,10 @@ constexpr int HT_WALK_NT = 128;
 
 // The count walk's output: the numbers of point-mass and cell entries.
 struct ListCount {
-    long long a = 0, b = 0;
+    int a = 0, b = 0;
     __device__ __forceinline__ void part(int) { a++; }
     __device__ __forceinline__ void parts(int, int n) { a += n; }
     __device__ __forceinline__ void cell(int) { b++; }
-    __device__ __forceinline__ void flush() {}
 };
 
 // One list of the fill walk, written in aligned 16-byte chunks: the entries of the current chunk
@@ -733,114 +752,81 @@ __device__ __forceinline__ bool take_node(const WalkNode& C, int w, const double
     return false;
 }
 
-// Depth-first walk below node v (descended into), children in octant order.  The nodes are in
-// pre-order, so the walk needs no stack: a node taken whole is followed by the node after its
-// subtree (w + nsub), a node descended into by its first child (w + 1), and the walk ends at
-// the end of v's subtree -- the same nodes in the same order as a recursive walk over the
-// children, one node record read per step.
+// Work unit u of the group with node gv.  The nodes are in pre-order, so the
+// depth-first walk (children in octant order) needs no stack: a node taken whole is followed by the
+// node after its subtree (w + nsub), a node descended into by its first child (w + 1), one node
+// record read per step.  A unit starts at its first node, unless the walk takes one of that node's
+// ancestors whole: then behind the subtree of the topmost such ancestor (which the unit that holds
+// its number emits).
+// The root: the group's list is the root as one cell when the root passes the opening test
+// (group_list of the host builder), the root's particles when it has at most nleaf particles or no
+// children.
 template <class ListOut>
-__device__ void walk_below(const Tree& T, const WalkNode* __restrict__ wn, int v, const double g[3], double h,
-                           double th2, ListOut& L) {
-    (void)T;
-    const int end = v + wn[v].nsub;
-    for (int w = v + 1; w < end;) {
+__device__ __forceinline__ void unit_walk(const Tree& T, const WalkNode* __restrict__ wn, const int* __restrict__ ppar,
+                                          Units U, int gv, int u, double th2, ListOut& L) {
+    const double g[3] = {T.c[3 * gv], T.c[3 * gv + 1], T.c[3 * gv + 2]};
+    const double h = T.half[gv];
+    const int end = U.begin(u + 1);
+    int w = U.begin(u);
+    if (w >= end) return;
+    const WalkNode R = wn[0];
+    const bool cell = !(dm(box_d2(R.com, g, h), th2) < R.side2);
+    if (cell || R.kind != WK_SPLIT) {
+        if (w > 0) return;
+        if (cell) L.cell(0);
+        else L.parts(R.first, R.count);
+        return;
+    }
+    int next = max(w, 1);
+    for (int a = w > 0 ? ppar[w] : 0; a > 0; a = ppar[a]) {
+        const WalkNode C = wn[a];
+        if (C.kind != WK_SPLIT || dm(box_d2(C.com, g, h), th2) > C.side2) next = a + C.nsub;
+    }
+    for (w = next; w < end;) {
         const WalkNode C = wn[w];
         w += take_node(C, w, g, h, th2, L) ? C.nsub : 1;
     }
 }
 
-// Work unit u of the group with node gv.  The root: the group's list is the root as one cell
-// when the root passes the opening test (group_list of the host builder), the root's particles
-// when it has at most nleaf particles or no children; unit 0 emits either.
-template <class ListOut>
-__device__ void unit_walk(const Tree& T, const WalkNode* __restrict__ wn, int gv, int u, double th2, ListOut& L) {
-    const double g[3] = {T.c[3 * gv], T.c[3 * gv + 1], T.c[3 * gv + 2]};
-    const double h = T.half[gv];
-    const WalkNode R = wn[0];
-    if (!(dm(box_d2(R.com, g, h), th2) < R.side2)) {
-        if (u == 0) L.cell(0);
-        return;
-    }
-    if (R.kind != WK_SPLIT) {
-        if (u == 0) L.parts(R.first, R.count);
-        return;
-    }
-    int v = 0; // a node the walk descends into
-#pragma unroll
-    for (int l = 1; l <= HT_UNIT_LEVELS; l++) {
-        const int below = 3 * (HT_UNIT_LEVELS - l);
-        const int c = T.child[8 * v + ((u >> below) & 7)];
-        if (c < 0) return;
-        const WalkNode C = wn[c];
-        if (l == HT_UNIT_LEVELS) {
-            if (!take_node(C, c, g, h, th2, L)) walk_below(T, wn, c, g, h, th2, L);
-            return;
-        }
-        if (C.kind != WK_SPLIT || dm(box_d2(C.com, g, h), th2) > C.side2) {
-            if ((u & ((1 << below) - 1)) == 0) take_node(C, c, g, h, th2, L);
-            return;
-        }
-        v = c;
-    }
-}
-
-// The unit whose node (HT_UNIT_LEVELS levels below the root) holds the group's node gv: its
-// octant digits from the centres, as the partition assigns them (a point above a node's centre
-// on an axis goes to the upper half).  A group above that depth takes the digits down to itself
-// and zeros below.
-__device__ __forceinline__ int home_unit(const Tree& T, int gv) {
-    const double cx = T.c[3 * gv], cy = T.c[3 * gv + 1], cz = T.c[3 * gv + 2];
-    int u = 0, v = 0;
-#pragma unroll
-    for (int l = 0; l < HT_UNIT_LEVELS; l++) {
-        int o = 0;
-        if (v >= 0 && v != gv) {
-            o = ((cx > T.c[3 * v]) << 2) | ((cy > T.c[3 * v + 1]) << 1) | (int)(cz > T.c[3 * v + 2]);
-            v = T.child[8 * v + o];
-        }
-        u = (u << 3) | o;
-    }
-    return u;
-}
-
 // Thread q takes rank q / ng of group q % ng: the lanes of a warp take the same rank of
 // neighbouring groups, whose walks are alike.  Rank r is unit r ^ home: rank 0 is the unit
-// around the group (the longest walk), ranks 1-7 its siblings, then the units under the other
-// children of the root -- so the long walks start first and the grid's last blocks are short.
-// Counts and offsets are stored group-major (g * HT_UNITS + u), the order of the lists.
-__global__ void __launch_bounds__(HT_WALK_NT) k_list_count(Tree T, const WalkNode* wn, const int* gnode, int ng,
-                                                          double th2, long long* np, long long* nc) {
+// around the group (the longest walk), the next ranks those beside it -- so the long walks start
+// first and the grid's last blocks are short.
+// Counts and offsets are stored group-major (g 2^ulog + u), the order of the lists.
+__global__ void __launch_bounds__(HT_WALK_NT) k_list_count(Tree T, const WalkNode* wn, const int* ppar, Units U,
+                                                          const int* gnode, int ng, double th2, long long* np,
+                                                          long long* nc) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (long long)ng * HT_UNITS) return;
+    if (q >= (long long)ng << U.ulog) return;
     const int g = (int)(q % ng), gv = gnode[g];
-    const int u = (int)(q / ng) ^ home_unit(T, gv);
+    const int u = (int)(q / ng) ^ U.of(gv);
     ListCount L;
-    unit_walk(T, wn, gv, u, th2, L);
-    np[(long long)g * HT_UNITS + u] = L.a;
-    nc[(long long)g * HT_UNITS + u] = L.b;
+    unit_walk(T, wn, ppar, U, gv, u, th2, L);
+    np[((long long)g << U.ulog) + u] = L.a;
+    nc[((long long)g << U.ulog) + u] = L.b;
 }
 
-__global__ void __launch_bounds__(HT_WALK_NT) k_list_fill(Tree T, const WalkNode* wn, const int* gnode, int ng,
-                                                         double th2, const long long* uoffp, const long long* uoffc,
+__global__ void __launch_bounds__(HT_WALK_NT) k_list_fill(Tree T, const WalkNode* wn, const int* ppar, Units U,
+                                                         const int* gnode, int ng, double th2, const long long* uoffp, const long long* uoffc,
                                                          int* pidx, int* cidx) {
     const long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (long long)ng * HT_UNITS) return;
+    if (q >= (long long)ng << U.ulog) return;
     const int g = (int)(q % ng), gv = gnode[g];
-    const int u = (int)(q / ng) ^ home_unit(T, gv);
-    const long long r = (long long)g * HT_UNITS + u;
+    const int u = (int)(q / ng) ^ U.of(gv);
+    const long long r = ((long long)g << U.ulog) + u;
     __shared__ int stage[2][4][HT_WALK_NT];
     ListFill L{ChunkOut(pidx + uoffp[r], &stage[0][0][threadIdx.x]), ChunkOut(cidx + uoffc[r], &stage[1][0][threadIdx.x])};
-    unit_walk(T, wn, gv, u, th2, L);
+    unit_walk(T, wn, ppar, U, gv, u, th2, L);
     L.flush();
 }
 
 // per-group offsets from the per-unit offsets (entry ng: the totals)
-__global__ void k_group_offsets(int ng, const long long* uoffp, const long long* uoffc, long long* poff,
+__global__ void k_group_offsets(int ng, int ulog, const long long* uoffp, const long long* uoffc, long long* poff,
                                 long long* coff) {
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g > ng) return;
-    poff[g] = uoffp[(long long)g * HT_UNITS];
-    coff[g] = uoffc[(long long)g * HT_UNITS];
+    poff[g] = uoffp[(long long)g << ulog];
+    coff[g] = uoffc[(long long)g << ulog];
 }
 
 __global__ void k_iota(int n, int* p) {
@@ -892,6 +878,14 @@ bool ensure_device() {
     PGB_CUDA_OR(g_err, LIB, cudaSetDevice(g_device), return false);
     return true;
 }
+
+// log2 of the list units a group: more of them shorten the longest walk (whose length goes as
+// theta^-3), fewer test fewer ancestors (at a unit's start; ng 2^ulog times) and keep fewer counts (32
+// bytes a unit).  Measured, count + fill (us) with 64 / 128 / 256 / 512 units, and with the 64 cells two
+// levels below the root: 2^20 Hernquist particles in 13880 groups, theta 0.5: 1715 / 1507 / 1213 / 1502
+// (2927); 2^22 in 55032: 3875 / 3799 / 4275 / 5507 (4710); 50000 in 1378: 275 / 165 / 124 / 144 (959); 2^18
+// in 13883, theta 0.75: 454 / 400 / 495 / 740 (684).
+int list_unit_log(int ng, double theta) { return ng <= 32768 && (double)ng * theta * theta * theta <= 2500.0 ? 8 : 7; }
 
 inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
@@ -1137,7 +1131,8 @@ bool build(pgbt_tree* T, const double* xh, const double* mh) {
 
     // interaction lists: count, prefix sums, fill
     DevBuf<long long>&unp = T->unp, &unc = T->unc, &uoffp = T->uoffp, &uoffc = T->uoffc;
-    const long long nu = (long long)ng * HT_UNITS;
+    const Units U{list_unit_log(ng, T->theta), nn};
+    const long long nu = (long long)ng << U.ulog;
     PGB_CUDA_OR(g_err, LIB, unp.reserve((size_t)nu + 1), return false);
     PGB_CUDA_OR(g_err, LIB, unc.reserve((size_t)nu + 1), return false);
     PGB_CUDA_OR(g_err, LIB, uoffp.reserve((size_t)nu + 1), return false);
@@ -1148,10 +1143,10 @@ bool build(pgbt_tree* T, const double* xh, const double* mh) {
     PGB_CUDA_OR(g_err, LIB, T->wn.reserve((size_t)nn * sizeof(WalkNode)), return false);
     WalkNode* wn = reinterpret_cast<WalkNode*>(T->wn.p);
     k_walk_nodes<<<nblk(nn, 256), 256, 0, s>>>(P, nn, T->nleaf, T->sizep.p, wn);
-    k_list_count<<<nblk(nu, HT_WALK_NT), HT_WALK_NT, 0, s>>>(P, wn, T->gnode.p, ng, th2, unp.p, unc.p);
+    k_list_count<<<nblk(nu, HT_WALK_NT), HT_WALK_NT, 0, s>>>(P, wn, T->ppar.p, U, T->gnode.p, ng, th2, unp.p, unc.p);
     if (!excl_scan<long long>(unp.p, nu, uoffp.p, s, ltmp)) return false;
     if (!excl_scan<long long>(unc.p, nu, uoffc.p, s, ltmp)) return false;
-    k_group_offsets<<<nblk((long long)ng + 1, 256), 256, 0, s>>>(ng, uoffp.p, uoffc.p, T->poff.p, T->coff.p);
+    k_group_offsets<<<nblk((long long)ng + 1, 256), 256, 0, s>>>(ng, U.ulog, uoffp.p, uoffc.p, T->poff.p, T->coff.p);
     long long tot[2] = {0, 0};
     if (!to_host(&tot[0], T->poff.p + ng, 1, s) || !to_host(&tot[1], T->coff.p + ng, 1, s)) return false;
     PGB_CUDA_OR(g_err, LIB, cudaStreamSynchronize(s), return false);
@@ -1159,7 +1154,7 @@ bool build(pgbt_tree* T, const double* xh, const double* mh) {
     T->nc = tot[1];
     PGB_CUDA_OR(g_err, LIB, T->pidx.reserve((size_t)std::max(1LL, T->np)), return false);
     PGB_CUDA_OR(g_err, LIB, T->cidx.reserve((size_t)std::max(1LL, T->nc)), return false);
-    k_list_fill<<<nblk(nu, HT_WALK_NT), HT_WALK_NT, 0, s>>>(P, wn, T->gnode.p, ng, th2, uoffp.p, uoffc.p, T->pidx.p, T->cidx.p);
+    k_list_fill<<<nblk(nu, HT_WALK_NT), HT_WALK_NT, 0, s>>>(P, wn, T->ppar.p, U, T->gnode.p, ng, th2, uoffp.p, uoffc.p, T->pidx.p, T->cidx.p);
     // force-launch records
     PGB_CUDA_OR(g_err, LIB, T->part.reserve((size_t)n), return false);
     PGB_CUDA_OR(g_err, LIB, T->cell.reserve((size_t)nn), return false);
