@@ -374,12 +374,14 @@ long long plan_items(std::vector<Task>& tasks, std::vector<Group>& groups, int& 
     for (int k = 0; k < nitem; k++) {
         int ni = items[4 * k + 1], nj = items[4 * k + 3];
         long long jc;
+        int align = K.paired ? K.tile : 1;
         if (nitem == 1) {
             // one item of equal tasks: the chunk count that minimises the wave quantisation, or
             // the autotuner's (nch_fixed)
             long long itiles = (ni + itile - 1) / itile;
             static const int forced_nch = env_int("PGB_G6_NCH", 0, 0, 4096);   // profiling: a pinned count
-            const int nch = forced_nch > 0 ? forced_nch : nch_fixed;
+            const int nch = forced_nch > 0 ? forced_nch : (nch_fixed < 0 ? -nch_fixed : nch_fixed);
+            if (nch_fixed < 0) align = 1;
             if (nch > 0) jc = (nj + nch - 1) / nch;
             else jc = model_chunk(K, itiles, nj, slots, (int)maxch);
         } else {
@@ -389,7 +391,7 @@ long long plan_items(std::vector<Task>& tasks, std::vector<Group>& groups, int& 
         }
         if (jc > nj) jc = nj > 0 ? nj : 1;
         rows += plan_item(tasks, groups, items[4 * k], ni, items[4 * k + 2], nj, itile, (int)jc, rows,
-                          K.paired ? K.tile : 1);
+                          align);
         inter += (long long)ni * nj;
     }
     std::stable_sort(tasks.begin(), tasks.end(), [](const Task& a, const Task& b) {
@@ -1139,7 +1141,7 @@ namespace {
 // two) and the variant flags, so plans of the same shape reuse a measured choice.
 std::mutex g_tune_mu;
 struct Tuned {
-    int cfg, nch;   // nch 0: the wave model's chunk count
+    int cfg, nch;   // nch 0: the model's chunk count; below 0: -nch chunks, not of whole tiles
 };
 std::vector<std::pair<long long, Tuned>> g_tune;
 
@@ -1427,7 +1429,13 @@ PGB_EXPORT int pgb6_plan_tune(pgb6_plan* P, const void* ipart, const void* jpred
             const KernelInfo K = kernel_info(cfg, P->ff, P->nn, false);
             const long long jc = model_chunk(K, (ni + K.itile - 1) / K.itile, nj, sm_count(g_device) * K.occ, maxch);
             const int m = (int)((nj + jc - 1) / jc);
-            for (int nch : chunk_candidates(m, nj, maxch)) {
+            std::vector<int> cand = chunk_candidates(m, nj, maxch);
+            // of whole tiles a j-paired kernel may have no count that fills one wave of CTAs: the wave
+            // model's, in plain chunks (3479 x 11705 without neighbours: 21 chunks of 557 records,
+            // 85.8 us, against 87.7 for the best of whole tiles)
+            if (K.paired)
+                cand.push_back(-best_nch((ni + K.itile - 1) / K.itile, nj, sm_count(g_device) * K.occ, maxch));
+            for (int nch : cand) {
                 if (nch == m) continue;   // timed above
                 float t;
                 if (!time_plan(cfg, nch, &t)) break;
