@@ -477,27 +477,46 @@ __global__ void __launch_bounds__(HT_NT) k_scatter_w(Nodes N, const int* tile_no
 
 // ---- pre-order numbering ------------------------------------------------------------------
 
-__global__ void k_subtree(Nodes N, int b, int e, int* size) {
-    const int v = b + blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= e) return;
-    int s = 1;
-    for (int o = 0; o < 8; o++) {
-        const int w = N.child[8 * v + o];
-        if (w >= 0) s += size[w];
+// Subtree sizes, and where each child's subtree starts behind its parent (off), bottom-up in one
+// launch: a thread per leaf climbs, and goes on from a node as its last child to arrive (done[], zero
+// at the start).  Nobody waits.
+__global__ void k_subtree(Nodes N, int nn, int* done, int* size, int* off) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= nn) return;
+    if (v == 0) off[0] = 0;
+    for (int o = 0; o < 8; o++)
+        if (N.child[8 * v + o] >= 0) return;
+    size[v] = 1;
+    for (int p = N.parent[v]; p >= 0; p = N.parent[p]) {
+        int w[8], kids = 0;
+#pragma unroll
+        for (int o = 0; o < 8; o++) {
+            w[o] = N.child[8 * p + o];
+            kids += w[o] >= 0;
+        }
+        __threadfence();
+        if (atomicAdd(done + p, 1) != kids - 1) return;
+        __threadfence();
+        int run = 1, sz[8];
+#pragma unroll
+        for (int o = 0; o < 8; o++) sz[o] = w[o] >= 0 ? __ldcg(size + w[o]) : 0;
+#pragma unroll
+        for (int o = 0; o < 8; o++)
+            if (w[o] >= 0) {
+                off[w[o]] = run;
+                run += sz[o];
+            }
+        size[p] = run;
     }
-    size[v] = s;
 }
 
-__global__ void k_preorder(Nodes N, int b, int e, const int* size, int* pre) {
-    const int v = b + blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= e) return;
-    int run = pre[v] + 1;
-    for (int o = 0; o < 8; o++) {
-        const int w = N.child[8 * v + o];
-        if (w < 0) continue;
-        pre[w] = run;
-        run += size[w];
-    }
+// Pre-order numbers: the sum of off up the path to the root.
+__global__ void k_preorder(Nodes N, int nn, const int* off, int* pre) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= nn) return;
+    int n = 0;
+    for (int a = v; a >= 0; a = N.parent[a]) n += off[a];
+    pre[v] = n;
 }
 
 struct Tree {   // pre-order output arrays
@@ -542,16 +561,25 @@ __device__ __forceinline__ void quad_add(double q[6], double m, const double d[3
     q[4] = da(q[4], dm(m, dm(dm(3.0, d[1]), d[2])));
 }
 
-// Moments of the nodes of one level (pre-order indices in `list`), children already done.
-__global__ void k_moments(Tree T, const int* list, int cnt, const double* xt, const double* mt) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cnt) return;
-    const int v = list[i];
-    bool leaf = true;
-    for (int o = 0; o < 8; o++) leaf = leaf && T.child[8 * v + o] < 0;
-    double m = 0.0, s[3] = {0.0, 0.0, 0.0}, q[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, com[3];
-    const int first = T.first[v], count = T.count[v];
-    if (leaf) {
+__device__ __forceinline__ void put_moments(const Tree& T, int v, double m, const double com[3], double q[6]) {
+    q[5] = -da(q[0], q[3]);
+    T.mass[v] = m;
+    for (int a = 0; a < 3; a++) T.com[3 * v + a] = com[a];
+    for (int k = 0; k < 6; k++) T.quad[6 * v + k] = q[k];
+}
+
+// Moments of every node in one launch: a thread per leaf sums its particles and climbs; of the
+// children of a node the one that finishes last (done[], zero at the start) combines all of them, in
+// octant order whoever it is, and climbs on.  Nobody waits.  154 us for the 17 levels of 2^20 Hernquist
+// particles; a launch per level, each as long as its slowest node, took 246.
+__global__ void k_moments(Tree T, const int* ppar, int nn, int* done, const double* xt, const double* mt) {
+    const int v = blockIdx.x * blockDim.x + threadIdx.x;
+    if (v >= nn) return;
+    for (int o = 0; o < 8; o++)
+        if (T.child[8 * v + o] >= 0) return;
+    {
+        double m = 0.0, s[3] = {0.0, 0.0, 0.0}, q[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, com[3];
+        const int first = T.first[v], count = T.count[v];
         for (int k = first; k < first + count; k++) {
             m = da(m, mt[k]);
             for (int a = 0; a < 3; a++) s[a] = da(s[a], dm(mt[k], xt[3 * (size_t)k + a]));
@@ -563,27 +591,43 @@ __global__ void k_moments(Tree T, const int* list, int cnt, const double* xt, co
                                      ds(xt[3 * (size_t)k + 2], com[2])};
                 quad_add(q, mt[k], d);
             }
-    } else {
-        for (int o = 0; o < 8; o++) {
-            const int w = T.child[8 * v + o];
-            if (w < 0) continue;
-            m = da(m, T.mass[w]);
-            for (int a = 0; a < 3; a++) s[a] = da(s[a], dm(T.mass[w], T.com[3 * w + a]));
-        }
-        for (int a = 0; a < 3; a++) com[a] = s[a] / m;
-        for (int o = 0; o < 8; o++) {
-            const int w = T.child[8 * v + o];
-            if (w < 0) continue;
-            const double d[3] = {ds(T.com[3 * w], com[0]), ds(T.com[3 * w + 1], com[1]), ds(T.com[3 * w + 2], com[2])};
-            quad_add(q, T.mass[w], d);
-            if (T.count[w] > 1)
-                for (int k = 0; k < 5; k++) q[k] = da(q[k], T.quad[6 * w + k]);
-        }
+        put_moments(T, v, m, com, q);
     }
-    q[5] = -da(q[0], q[3]);
-    T.mass[v] = m;
-    for (int a = 0; a < 3; a++) T.com[3 * v + a] = com[a];
-    for (int k = 0; k < 6; k++) T.quad[6 * v + k] = q[k];
+    for (int p = ppar[v]; p >= 0; p = ppar[p]) {
+        int w[8], kids = 0;
+#pragma unroll
+        for (int o = 0; o < 8; o++) {
+            w[o] = T.child[8 * p + o];
+            kids += w[o] >= 0;
+        }
+        __threadfence();
+        if (atomicAdd(done + p, 1) != kids - 1) return;
+        __threadfence();
+        double m = 0.0, s[3] = {0.0, 0.0, 0.0}, q[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, com[3];
+        double mw[8], cw[8][3];   // the children's, from L2: other SMs have written them
+#pragma unroll
+        for (int o = 0; o < 8; o++)
+            if (w[o] >= 0) {
+                mw[o] = __ldcg(T.mass + w[o]);
+                for (int a = 0; a < 3; a++) cw[o][a] = __ldcg(T.com + 3 * w[o] + a);
+            }
+#pragma unroll
+        for (int o = 0; o < 8; o++)
+            if (w[o] >= 0) {
+                m = da(m, mw[o]);
+                for (int a = 0; a < 3; a++) s[a] = da(s[a], dm(mw[o], cw[o][a]));
+            }
+        for (int a = 0; a < 3; a++) com[a] = s[a] / m;
+#pragma unroll
+        for (int o = 0; o < 8; o++)
+            if (w[o] >= 0) {
+                const double d[3] = {ds(cw[o][0], com[0]), ds(cw[o][1], com[1]), ds(cw[o][2], com[2])};
+                quad_add(q, mw[o], d);
+                if (T.count[w[o]] > 1)
+                    for (int k = 0; k < 5; k++) q[k] = da(q[k], __ldcg(T.quad + 6 * w[o] + k));
+            }
+        put_moments(T, p, m, com, q);
+    }
 }
 
 // ---- groups and lists ---------------------------------------------------------------------
@@ -915,7 +959,7 @@ struct pgbt_tree {
     DevBuf<unsigned long long> mx;
     DevBuf<int> ntile, tile_off, tile_node, tcount, tbase, ccount, nkids, kid_off;
     DevBuf<unsigned char> oct;
-    DevBuf<int> size, pre, lvl_pre, gflag, goff;
+    DevBuf<int> size, pre, gflag, goff;
     DevBuf<int> sizep;   // subtree sizes (nodes) in pre-order, for the stackless list walks
     DevBuf<long long> unp, unc, uoffp, uoffc;
     DevBuf<unsigned char> wn;   // WalkNode records
@@ -1078,15 +1122,16 @@ bool build(pgbt_tree* T, const double* xh, const double* mh) {
     T->nn = nn;
     Nodes N = bfs(T);
 
-    // pre-order numbering: subtree sizes bottom-up, numbers top-down
-    DevBuf<int>&size = T->size, &pre = T->pre;
+    // pre-order numbering; the nodes' counters and offsets lie where the group flags and their scan go
+    // afterwards
+    DevBuf<int>&size = T->size, &pre = T->pre, &gflag = T->gflag, &goff = T->goff;
     PGB_CUDA_OR(g_err, LIB, size.reserve((size_t)nn), return false);
     PGB_CUDA_OR(g_err, LIB, pre.reserve((size_t)nn), return false);
-    for (int L = nlev - 1; L >= 0; L--)
-        if (lvl[L + 1] > lvl[L]) k_subtree<<<nblk(lvl[L + 1] - lvl[L], 256), 256, 0, s>>>(N, lvl[L], lvl[L + 1], size.p);
-    PGB_CUDA_OR(g_err, LIB, cudaMemsetAsync(pre.p, 0, sizeof(int), s), return false);
-    for (int L = 0; L < nlev; L++)
-        if (lvl[L + 1] > lvl[L]) k_preorder<<<nblk(lvl[L + 1] - lvl[L], 256), 256, 0, s>>>(N, lvl[L], lvl[L + 1], size.p, pre.p);
+    PGB_CUDA_OR(g_err, LIB, gflag.reserve((size_t)nn), return false);
+    PGB_CUDA_OR(g_err, LIB, goff.reserve((size_t)nn + 1), return false);
+    PGB_CUDA_OR(g_err, LIB, cudaMemsetAsync(gflag.p, 0, (size_t)nn * sizeof(int), s), return false);
+    k_subtree<<<nblk(nn, 256), 256, 0, s>>>(N, nn, gflag.p, size.p, goff.p);
+    k_preorder<<<nblk(nn, 256), 256, 0, s>>>(N, nn, goff.p, pre.p);
     PGB_CUDA_OR(g_err, LIB, T->first.reserve((size_t)nn), return false);
     PGB_CUDA_OR(g_err, LIB, T->count.reserve((size_t)nn), return false);
     PGB_CUDA_OR(g_err, LIB, T->child.reserve(8 * (size_t)nn), return false);
@@ -1105,21 +1150,12 @@ bool build(pgbt_tree* T, const double* xh, const double* mh) {
     PGB_CUDA_OR(g_err, LIB, T->mt.reserve((size_t)n), return false);
     k_gather<<<nblk(n, 256), 256, 0, s>>>(n, T->perm.p, T->x.p, T->m.p, T->xt.p, T->mt.p);
 
-    // moments, deepest level first: the pre-order indices of each level
-    DevBuf<int>& lvl_pre = T->lvl_pre;
-    PGB_CUDA_OR(g_err, LIB, lvl_pre.reserve((size_t)nn), return false);
-    PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(lvl_pre.p, pre.p, (size_t)nn * sizeof(int), cudaMemcpyDeviceToDevice, s),
-                return false);
-    for (int L = nlev - 1; L >= 0; L--) {
-        const int cnt = lvl[L + 1] - lvl[L];
-        if (cnt > 0) k_moments<<<nblk(cnt, 128), 128, 0, s>>>(P, lvl_pre.p + lvl[L], cnt, T->xt.p, T->mt.p);
-    }
+    // moments, with the same counters
+    k_parent_pre<<<nblk(nn, 256), 256, 0, s>>>(P, nn, T->ppar.p);
+    PGB_CUDA_OR(g_err, LIB, cudaMemsetAsync(gflag.p, 0, (size_t)nn * sizeof(int), s), return false);
+    k_moments<<<nblk(nn, 128), 128, 0, s>>>(P, T->ppar.p, nn, gflag.p, T->xt.p, T->mt.p);
 
     // groups in pre-order
-    k_parent_pre<<<nblk(nn, 256), 256, 0, s>>>(P, nn, T->ppar.p);
-    DevBuf<int>&gflag = T->gflag, &goff = T->goff;
-    PGB_CUDA_OR(g_err, LIB, gflag.reserve((size_t)nn), return false);
-    PGB_CUDA_OR(g_err, LIB, goff.reserve((size_t)nn + 1), return false);
     k_group_flags<<<nblk(nn, 256), 256, 0, s>>>(P, T->ppar.p, nn, T->ncrit, gflag.p);
     if (!excl_scan<int>(gflag.p, nn, goff.p, s, stmp)) return false;
     int ng = 0;
@@ -1186,7 +1222,7 @@ void tree_free(pgbt_tree* T) {
     for (auto& b : T->ltmp) b.release();
     T->mx.release();
     DevBuf<int>* sc[] = {&T->ntile, &T->tile_off, &T->tile_node, &T->tcount, &T->tbase, &T->ccount, &T->nkids,
-                         &T->kid_off, &T->size, &T->pre, &T->lvl_pre, &T->gflag, &T->goff, &T->sizep};
+                         &T->kid_off, &T->size, &T->pre, &T->gflag, &T->goff, &T->sizep};
     for (auto* b : sc) b->release();
     T->oct.release();
     T->wn.release();
