@@ -53,10 +53,12 @@ SM_COUNT = 148
 REF_SRC = os.environ.get("PGB_REFERENCE", "/root/reference")
 # DRAM bytes (read + write) of one launch of the roofline kernel, from the committed ncu captures
 # (dram__bytes_read.sum + dram__bytes_write.sum); the bench cannot run ncu itself.
-G6_CFG_NAMES = ["512x1 (8 j-lanes)", "256x1 (2 j-lanes)", "128x2 i-paired", "128x1", "128x4 i-paired",
+G6_CFG_NAMES = ["512x1 (8 j-lanes)", "128x2 j-paired (2 j-lanes, best quad)", "128x2 i-paired",
+                "128x2 j-paired (best quad)", "128x4 i-paired",
                 "256x2 i-paired", "128x2 j-paired", "256x2 j-paired", "128x4 j-paired",
                 "128x2 j-paired stage-ordered"]   # pgb6 configurations
-G5_CFG_NAMES = ["128x4", "256x2", "512x2", "1024x1", "384x2", "128x2", "128x1", "64x1", "64x1 j-paired",
+G5_CFG_NAMES = ["128x4", "256x2", "512x2", "1024x1", "384x2", "128x2", "128x1", "64x1 (16 i-slots x 4 j-lanes)",
+                "64x1 (16 i-slots x 4 j-lanes)",
                 "1024x1 j-paired", "256x1 j-paired"]   # pgb5 configurations (threads x i/thread)
 PROFILED_TRAFFIC = {
     # the largest Hermite call by the configuration that runs it (6: 128x2 j-paired, 2: 128x2 i-paired)

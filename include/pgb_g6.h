@@ -169,7 +169,7 @@ int  pgb6_hermite_step(pgb6_hermite *h, double *time, int *ni);
 /* block steps while the global time is below tend; steps taken by this call (optional) */
 int  pgb6_hermite_advance(pgb6_hermite *h, double tend, long long *psteps, long long *bsteps);
 double pgb6_hermite_time(pgb6_hermite *h);
-/* Fault handling of the step kernel: every wait (grid barrier, segment / task flag) gives up
+/* Fault handling of the step kernel: every wait (segment record, chunk sums, segment / task flag) gives up
  * after a limit of SM cycles (default about a second; cycles <= 0 restores it), after which
  * every CTA returns, the call reports PGB_ERR_DEVICE and the integrator is unusable.
  * wait_status reads whether a wait gave up, how many CTAs have returned from the kernel (over

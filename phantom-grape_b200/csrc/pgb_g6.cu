@@ -1112,7 +1112,8 @@ PGB_EXPORT void pgb6_set_abort(int on) {
 // Sizes of the device record types, so callers can lay out device buffers:
 // G6Ptcl (j-memory), G6PredJ (predicted j), G6I (i-particle), G6Out (result).
 // Device-time accounting of the drop-in calls (no counterpart in the reference): with on != 0,
-// every g6calc_firsthalf (j-memory update + prediction) and g6calc_lasthalf* (force launch)
+// every g6calc_firsthalf (j-memory update + prediction) and g6calc_lasthalf* (force launch, with the
+// sort of a small call's neighbour lists)
 // adds the device time between CUDA events recorded around its work on the library's stream
 // to a running total; pgb6_call_device_ms returns that total in ms (and clears it when reset
 // != 0).  It separates the device work of the plain API from its host overhead.
