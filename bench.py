@@ -70,10 +70,10 @@ PROFILED_TRAFFIC = {
                      "source": "profiles/g6_kernel_hermite_65536x65536.md (128x2 i-paired)"},
     "direct": {"bytes": 540_928, "pairs": 268_435_456,
                "source": "profiles/g5_kernels_direct_treepm_bh.md (1024x1 j-paired)"},
-    "treepm": {"bytes": 557_901_056 + 35_891_456, "pairs": 4_463_983_086,
+    "treepm": {"bytes": 556_061_184 + 35_729_664, "pairs": 4_463_983_086,
                "source": "profiles/g5_kernels_direct_treepm_bh.md (64x1)"},
     # captured at N = 2^20 (both launches of a step); scaled to the run's pairs
-    "bh": {"bytes": 131_828_224 + 26_739_456 + 227_582_208 + 31_331_072, "pairs": 4_462_862_693,
+    "bh": {"bytes": 132_578_816 + 25_789_440 + 228_481_792 + 31_241_472, "pairs": 4_462_862_693,
            "source": "profiles/g5_kernels_direct_treepm_bh.md (64x1, N=2^20 capture scaled by pairs)"},
 }
 

@@ -605,7 +605,7 @@ __global__ void __launch_bounds__(NT) g5_kernel(G5Args A) {
 // scalar chains): cells of an N = 2^20 tree 4156 -> 3563 us (799 Gint/s: with the idle slots 79 %
 // of the FMA rate), its point masses 974 -> 831 us (1930 Gint/s), the 4096 TreePM groups of 2^20
 // particles 2906 -> 2282 us (1955 Gint/s; 12 FMA operations, 4 integer ones and a table look-up of
-// 2.2 shared wavefronts a pair: FMA heavy half 70 %, shared wavefronts 60 %, issue 62 % busy).
+// 2.2 shared wavefronts a pair: FMA heavy half 65 %, shared wavefronts 70 %, issue 65 % busy).
 // A j-tile is G5S_NJ records as field arrays; lane l takes the tile's j-quads l, l + 4, ....  The
 // tile is padded to a multiple of 4 with massless records far away (G5S_FAR), which add exact
 // zeros to any finite sum.  FP32 sums cover a tile (32 terms a lane half and i at most), then go
