@@ -450,7 +450,6 @@ __device__ __forceinline__ void g6_jpair(float2 xh, float2 yh, float2 zh, float2
     const float2 r2v = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __ffma2_rn(dx, dx, make_float2(eps2, eps2))));
     const float2 rvv = __ffma2_rn(dz, dvz, __ffma2_rn(dy, dvy, __fmul2_rn(dx, dvx)));
     float2 sv;
-    const float* mp = &m.x;
     const int* idp = &jid.x;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
