@@ -445,9 +445,10 @@ __global__ void __launch_bounds__(NT) g5_kernel(G5Args A) {
     }
     const int tid = (int)threadIdx.x;
 
-    // The j-paired task: one i per thread.  The tile is staged as field arrays padded to a
-    // multiple of 4 with massless copies of its first record (and zero moments for cells), which
-    // add exact zeros.  FP32 sums are folded into FP64 every G5_FOLD j.
+    // The j-paired task: one i per thread.  The tile is staged as field arrays, whose whole quads are
+    // taken two j-pairs at a time and the records of a last, partial quad one by one, in both halves
+    // of sums of which one counts (padded with massless copies of a record instead, an unsoftened
+    // i on that record got 0 * inf).  FP32 sums are folded into FP64 every G5_FOLD j.
     auto jp_task = [&](const Task& T, double (&S)[4]) {
         G5TileSoA<NT>* sa = reinterpret_cast<G5TileSoA<NT>*>(sj);
         const float4 p = A.ipos[T.i0 + (tid < T.ni ? tid : 0)];
@@ -455,31 +456,29 @@ __global__ void __launch_bounds__(NT) g5_kernel(G5Args A) {
         const float2 ei = make_float2(p.w, p.w);
         for (int jt = 0; jt < T.nj; jt += NT) {
             const int nt = min(NT, T.nj - jt);
-            const int nt4 = (nt + 3) & ~3;
             __syncthreads();
-            if (tid < nt4) {
-                const bool real = tid < nt;
-                const int jk = T.j0 + jt + (real ? tid : 0);
+            if (tid < nt) {
+                const int jk = T.j0 + jt + tid;
                 const int jj = A.jidx ? __ldg(A.jidx + jk) : jk;
                 const float4 J = A.jpos[jj];
                 sa->x[tid] = J.x;
                 sa->y[tid] = J.y;
                 sa->z[tid] = J.z;
-                sa->m[tid] = real ? J.w : 0.0f;
+                sa->m[tid] = J.w;
                 if constexpr (KIND == G5_QUAD) {
                     const float4 Q0 = A.jaux[2 * jj], Q1 = A.jaux[2 * jj + 1];
-                    const float f = real ? G5_QSCALE : 0.0f;
-                    sa->q[0][tid] = f * Q0.x;
-                    sa->q[1][tid] = f * Q0.y;
-                    sa->q[2][tid] = f * Q0.z;
-                    sa->q[3][tid] = f * Q0.w;
-                    sa->q[4][tid] = f * Q1.x;
-                    sa->q[5][tid] = f * Q1.y;
+                    sa->q[0][tid] = G5_QSCALE * Q0.x;
+                    sa->q[1][tid] = G5_QSCALE * Q0.y;
+                    sa->q[2][tid] = G5_QSCALE * Q0.z;
+                    sa->q[3][tid] = G5_QSCALE * Q0.w;
+                    sa->q[4][tid] = G5_QSCALE * Q1.x;
+                    sa->q[5][tid] = G5_QSCALE * Q1.y;
                 }
             }
             __syncthreads();
-            for (int jb = 0; jb < nt4; jb += G5_FOLD) {
-                const int je = min(jb + G5_FOLD, nt4);
+            const int ntf = nt & ~3;
+            for (int jb = 0; jb < ntf; jb += G5_FOLD) {
+                const int je = min(jb + G5_FOLD, ntf);
                 float2 a2[NAcc<KIND>::n];
 #pragma unroll
                 for (int c = 0; c < NAcc<KIND>::n; c++) a2[c] = make_float2(0.f, 0.f);
@@ -508,6 +507,24 @@ __global__ void __launch_bounds__(NT) g5_kernel(G5Args A) {
                     }
                 }
                 g5_fold2<KIND>(S, a2, -1);
+            }
+            if (ntf < nt) {
+                float2 a2[NAcc<KIND>::n];
+#pragma unroll
+                for (int c = 0; c < NAcc<KIND>::n; c++) a2[c] = make_float2(0.f, 0.f);
+#pragma unroll 1
+                for (int j = ntf; j < nt; j++) {
+                    auto both = [&](const float* f) { return make_float2(f[j], f[j]); };
+                    if constexpr (KIND == G5_QUAD) {
+                        float2 Q[6];
+#pragma unroll
+                        for (int c = 0; c < 6; c++) Q[c] = both(sa->q[c]);
+                        g5_quad_jpair(both(sa->x), both(sa->y), both(sa->z), both(sa->m), Q, nx, ny, nz, ei, a2);
+                    } else {
+                        g5_newton_jpair(both(sa->x), both(sa->y), both(sa->z), both(sa->m), nx, ny, nz, ei, a2);
+                    }
+                }
+                g5_fold2<KIND>(S, a2, 0);
             }
         }
     };
