@@ -329,6 +329,13 @@ __device__ __forceinline__ void g5_quad_jpair(float2 X, float2 Y, float2 Z, floa
     a[4] = __ffma2_rn(p, D, a[4]);
 }
 
+// Half `second` of the sums t into a.
+template <int N>
+__device__ __forceinline__ void g5_half(float2 (&a)[N], const float2 (&t)[N], int second) {
+#pragma unroll
+    for (int c = 0; c < N; c++) a[c] = second ? make_float2(a[c].x, t[c].y) : make_float2(t[c].x, a[c].y);
+}
+
 // Final scaling of the FP64 sums into (acc, pot_raw).
 template <int KIND>
 __device__ __forceinline__ double4 g5_finish(double4 s, double ascale) {
@@ -624,8 +631,9 @@ __global__ void __launch_bounds__(NT) g5_kernel(G5Args A) {
 // particles 2906 -> 2282 us (1955 Gint/s; 12 FMA operations, 4 integer ones and a table look-up of
 // 2.2 shared wavefronts a pair: FMA heavy half 65 %, shared wavefronts 70 %, issue 65 % busy).
 // A j-tile is G5S_NJ records as field arrays; lane l takes the tile's j-quads l, l + 4, ....  The
-// tile is padded to a multiple of 4 with massless records far away (G5S_FAR), which add exact
-// zeros to any finite sum.  FP32 sums cover a tile (32 terms a lane half and i at most), then go
+// records of a last, partial quad are taken one by one (padded with massless records far away
+// instead, the padding's overflowed r^2 made its terms NaN with the Newton-refined rsqrt).
+// FP32 sums cover a tile (32 terms a lane half and i at most), then go
 // into the FP64 sums; the lanes' sums are added in lane order at the end of the task.
 constexpr int G5S_NT = 64, G5S_SLOTS = 16, G5S_LANES = 4, G5S_IPT = 4;
 constexpr int G5S_NJ = 256;   // records a tile: 64 a lane between two folds into FP64 (128: cells 3 % slower)
@@ -633,7 +641,6 @@ constexpr int G5S_NJ = 256;   // records a tile: 64 a lane between two folds int
 // registers, which reload the j fields per pair, 3639), point masses and the table 10 (95 registers)
 template <int KIND>
 constexpr int g5s_min_ctas() { return KIND == G5_QUAD ? 5 : 10; }
-constexpr float G5S_FAR = 1e18f;   // its square times three is finite
 
 template <int KIND>
 struct G5STile {
@@ -677,14 +684,14 @@ __device__ __forceinline__ void g5_slots_task(const G5Args& A, const Task& T, G5
     };
     load_idx(0);
     for (int jt = 0; jt < T.nj; jt += NJ) {
-        const int nt = min(NJ, T.nj - jt), nq = (nt + 3) >> 2;
+        const int nt = min(NJ, T.nj - jt), whole = nt >> 2;
         float4 J[R];
         float4 Q0[R], Q1[R];
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const int q = tid + r * G5S_NT;
-            J[r] = make_float4(G5S_FAR, G5S_FAR, G5S_FAR, 0.f);
-            Q0[r] = Q1[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+            // (a value for every thread: without it ptxas spills 200 to 480 bytes)
+            J[r] = Q0[r] = Q1[r] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (q < nt) {
                 const int jj = jn[r];
                 J[r] = A.jpos[jj];
@@ -699,7 +706,7 @@ __device__ __forceinline__ void g5_slots_task(const G5Args& A, const Task& T, G5
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const int q = tid + r * G5S_NT;
-            if (q < 4 * nq) {
+            if (q < nt) {
                 float(*f)[NJ] = sh.t.f;
                 f[0][q] = J[r].x;
                 f[1][q] = J[r].y;
@@ -723,8 +730,21 @@ __device__ __forceinline__ void g5_slots_task(const G5Args& A, const Task& T, G5
         for (int k = 0; k < IPT; k++)
 #pragma unroll
             for (int c = 0; c < NAcc<KIND>::n; c++) a[k][c] = make_float2(0.f, 0.f);
+        // the pair terms of i k and the two records w
+        auto add = [&](int k, const float2 (&w)[4 + G5STile<KIND>::NQ], float2 (&s)[NAcc<KIND>::n]) {
+            if constexpr (KIND == G5_QUAD) {
+                const float2 q[6] = {w[4], w[5], w[6], w[7], w[8], w[9]};
+                g5_quad_jpair(w[0], w[1], w[2], w[3], q, nx[k], ny[k], nz[k], ei[k], s);
+            } else if constexpr (KIND == G5_TABLE) {
+                g5_table_jpair(w[0], w[1], w[2], w[3], nx[k], ny[k], nz[k], tab, shift3, nodemask, A.r2cut, s);
+            } else if constexpr (KIND == G5_SYMMETRIC) {
+                g5_newton_jpair(w[0], w[1], w[2], w[3], nx[k], ny[k], nz[k], __fadd2_rn(ei[k], w[4]), s);
+            } else {
+                g5_newton_jpair(w[0], w[1], w[2], w[3], nx[k], ny[k], nz[k], ei[k], s);
+            }
+        };
 #pragma unroll 1
-        for (int jq = lane; jq < nq; jq += G5S_LANES) {
+        for (int jq = lane; jq < whole; jq += G5S_LANES) {
             float4 v[4 + G5STile<KIND>::NQ];
 #pragma unroll
             for (int c = 0; c < 4 + G5STile<KIND>::NQ; c++) v[c] = *reinterpret_cast<const float4*>(&sh.t.f[c][4 * jq]);
@@ -735,17 +755,22 @@ __device__ __forceinline__ void g5_slots_task(const G5Args& A, const Task& T, G5
                 for (int c = 0; c < 4 + G5STile<KIND>::NQ; c++)
                     w[c] = h ? make_float2(v[c].z, v[c].w) : make_float2(v[c].x, v[c].y);
 #pragma unroll
+                for (int k = 0; k < IPT; k++) add(k, w, a[k]);
+            }
+        }
+        if (lane == whole % G5S_LANES) {
+#pragma unroll 1
+            for (int j = 4 * whole; j < nt; j++) {
+                float2 w[4 + G5STile<KIND>::NQ];
+#pragma unroll
+                for (int c = 0; c < 4 + G5STile<KIND>::NQ; c++) w[c] = make_float2(sh.t.f[c][j], sh.t.f[c][j]);
+#pragma unroll
                 for (int k = 0; k < IPT; k++) {
-                    if constexpr (KIND == G5_QUAD) {
-                        const float2 q[6] = {w[4], w[5], w[6], w[7], w[8], w[9]};
-                        g5_quad_jpair(w[0], w[1], w[2], w[3], q, nx[k], ny[k], nz[k], ei[k], a[k]);
-                    } else if constexpr (KIND == G5_TABLE) {
-                        g5_table_jpair(w[0], w[1], w[2], w[3], nx[k], ny[k], nz[k], tab, shift3, nodemask, A.r2cut, a[k]);
-                    } else if constexpr (KIND == G5_SYMMETRIC) {
-                        g5_newton_jpair(w[0], w[1], w[2], w[3], nx[k], ny[k], nz[k], __fadd2_rn(ei[k], w[4]), a[k]);
-                    } else {
-                        g5_newton_jpair(w[0], w[1], w[2], w[3], nx[k], ny[k], nz[k], ei[k], a[k]);
-                    }
+                    float2 t[NAcc<KIND>::n];
+#pragma unroll
+                    for (int c = 0; c < NAcc<KIND>::n; c++) t[c] = a[k][c];
+                    add(k, w, t);
+                    g5_half(a[k], t, j & 1);
                 }
             }
         }
