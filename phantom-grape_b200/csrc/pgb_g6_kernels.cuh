@@ -421,7 +421,9 @@ __device__ __forceinline__ void g6_pair2(const G6PredJ& J, int jadr, const Pos3*
 // differences scalar too and 5.10 ms with the relative coordinates scalar also.
 // The two lanes of each accumulator sum the even and the odd j of the tile; they are added
 // into the FP64 sums one after the other at every fold.  Per pair the key q is bit-identical
-// to g6_key (FADD2 rounds each lane as FADD does).
+// to g6_key (FADD2 rounds each lane as FADD does).  live: how many of the records, from the first,
+// are the caller's (SELF only; a partial tile's last quad holds padding after them, whose pairs
+// are masked as self pairs are: massless copies alone give 0 * inf for an unsoftened pair at zero distance).
 struct G6IPair {
     float2 nxh, nyh, nzh, nxl, nyl, nzl;   // -x_i (hi, lo) of each coordinate, in both lanes
     float vx, vy, vz;
@@ -437,7 +439,7 @@ struct G6TileSoA {
 
 template <bool NN, bool SELF>
 __device__ __forceinline__ void g6_jpair(float2 xh, float2 yh, float2 zh, float2 xl, float2 yl, float2 zl,
-                                         float2 m, float2 vx, float2 vy, float2 vz, int2 jid,
+                                         float2 m, float2 vx, float2 vy, float2 vz, int2 jid, int live,
                                          const G6IPair& I, float eps2, G6Acc2& a, float& tmin) {
     const float2 dx = __fadd2_rn(__fadd2_rn(xh, I.nxh), __fadd2_rn(xl, I.nxl));
     const float2 dy = __fadd2_rn(__fadd2_rn(yh, I.nyh), __fadd2_rn(yl, I.nyl));
@@ -454,7 +456,7 @@ __device__ __forceinline__ void g6_jpair(float2 xh, float2 yh, float2 zh, float2
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         float s = pair_scale((&r2v.x)[h]);
-        if constexpr (SELF) s = (idp[h] == I.id) ? 0.0f : s;
+        if constexpr (SELF) s = (idp[h] == I.id || h >= live) ? 0.0f : s;
         if constexpr (NN) tmin = fminf(tmin, nn_key(s));
         (&sv.x)[h] = s;
     }
@@ -484,8 +486,8 @@ __device__ __forceinline__ void g6_jpair(float2 xh, float2 yh, float2 zh, float2
 template <bool NN, bool SELF>
 __device__ __forceinline__ void g6_jquad2(const float4& XH, const float4& YH, const float4& ZH, const float4& XL,
                                           const float4& YL, const float4& ZL, const float4& M, const float4& VX,
-                                          const float4& VY, const float4& VZ, const int4& ID, const G6IPair* IP,
-                                          float eps2, G6Acc2* a, float* tmin) {
+                                          const float4& VY, const float4& VZ, const int4& ID, int live,
+                                          const G6IPair* IP, float eps2, G6Acc2* a, float* tmin) {
     float2 dx[4], dy[4], dz[4];
 #pragma unroll
     for (int c = 0; c < 4; c++) {
@@ -538,7 +540,7 @@ __device__ __forceinline__ void g6_jquad2(const float4& XH, const float4& YH, co
         const G6IPair& I = IP[c >> 1];
         const int jj = ((c & 1) << 1) + h;
         float s = pair_scale_from_rsqrt(r2[l], y[l]);
-        if constexpr (SELF) s = (ids[jj] == I.id) ? 0.0f : s;
+        if constexpr (SELF) s = (ids[jj] == I.id || jj >= live) ? 0.0f : s;
         if constexpr (NN) tmin[c >> 1] = fminf(tmin[c >> 1], nn_key(s));
         sv[l] = s;
     }
@@ -873,8 +875,8 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
         bool mine = false;
         int nt4 = nt;
         if constexpr (USE_JP) {
-            // fields of the tile's records, padded to a multiple of 4 with massless copies of
-            // the tile's first record (they add exact zeros, and their key repeats that record's)
+            // fields of the tile's records, padded to a multiple of 4 with copies of the tile's
+            // first record (whose pairs are masked)
             nt4 = (nt + 3) & ~3;
 #pragma unroll
             for (int q = threadIdx.x; q < NJ; q += NT) {
@@ -887,7 +889,7 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
                 sa->xl[q] = r.p.f.xl;
                 sa->yl[q] = r.p.f.yl;
                 sa->zl[q] = r.p.f.zl;
-                sa->m[q] = real ? r.m : 0.0f;
+                sa->m[q] = r.m;
                 sa->vx[q] = r.vx;
                 sa->vy[q] = r.vy;
                 sa->vz[q] = r.vz;
@@ -939,7 +941,7 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
 #pragma unroll
                         for (int k = 0; k < IPT; k++) tq[k] = QUADMIN ? kmin[k] : tmin[k];
                         if constexpr (JP == 2 && IPT == 2) {
-                            g6_jquad2<NN, SELF>(XH, YH, ZH, XL, YL, ZL, M, VX, VY, VZ, ID, IP, A.eps2, a, tq);
+                            g6_jquad2<NN, SELF>(XH, YH, ZH, XL, YL, ZL, M, VX, VY, VZ, ID, nt - j, IP, A.eps2, a, tq);
                         } else {
 #pragma unroll
                         for (int k = 0; k < IPT; k++) {
@@ -948,13 +950,13 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
                                                make_float2(YL.x, YL.y), make_float2(ZL.x, ZL.y),
                                                make_float2(M.x, M.y), make_float2(VX.x, VX.y),
                                                make_float2(VY.x, VY.y), make_float2(VZ.x, VZ.y),
-                                               make_int2(ID.x, ID.y), IP[k], A.eps2, a[k], tq[k]);
+                                               make_int2(ID.x, ID.y), nt - j, IP[k], A.eps2, a[k], tq[k]);
                             g6_jpair<NN, SELF>(make_float2(XH.z, XH.w), make_float2(YH.z, YH.w),
                                                make_float2(ZH.z, ZH.w), make_float2(XL.z, XL.w),
                                                make_float2(YL.z, YL.w), make_float2(ZL.z, ZL.w),
                                                make_float2(M.z, M.w), make_float2(VX.z, VX.w),
                                                make_float2(VY.z, VY.w), make_float2(VZ.z, VZ.w),
-                                               make_int2(ID.z, ID.w), IP[k], A.eps2, a[k], tq[k]);
+                                               make_int2(ID.z, ID.w), nt - j - 2, IP[k], A.eps2, a[k], tq[k]);
                         }
                         }
                         if constexpr (NN) {

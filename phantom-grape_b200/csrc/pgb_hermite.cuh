@@ -688,7 +688,7 @@ __device__ __forceinline__ void hm_lanes(const unsigned char* smem, int nt, cons
         for (int j = 2 * p; j < nt; j += JL)
             g6_jpair<false, true>(f2(t->xh + j), f2(t->yh + j), f2(t->zh + j), f2(t->xl + j), f2(t->yl + j), f2(t->zl + j),
                                   f2(t->m + j), f2(t->vx + j), f2(t->vy + j), f2(t->vz + j),
-                                  *reinterpret_cast<const int2*>(t->id + j), IP, eps2, a, tmin);
+                                  *reinterpret_cast<const int2*>(t->id + j), 2, IP, eps2, a, tmin);
         const float2* v = &a.ax;
 #pragma unroll
         for (int q = 0; q < 6; q++) {

@@ -149,18 +149,18 @@ __global__ void __launch_bounds__(LOOP_NT) g6_loop_kernel(double* out, int passe
             const float4 VZ = *reinterpret_cast<const float4*>(&tile.vz[j]);
             const int4 ID = make_int4(0, 0, 0, 0);
             if constexpr (JP == 2) {
-                pgb::g6_jquad2<true, false>(XH, YH, ZH, XL, YL, ZL, M, VX, VY, VZ, ID, IP, eps2, a, tmin);
+                pgb::g6_jquad2<true, false>(XH, YH, ZH, XL, YL, ZL, M, VX, VY, VZ, ID, 4, IP, eps2, a, tmin);
             } else {
 #pragma unroll
                 for (int k = 0; k < 2; k++) {
                     pgb::g6_jpair<true, false>(make_float2(XH.x, XH.y), make_float2(YH.x, YH.y), make_float2(ZH.x, ZH.y),
                                                make_float2(XL.x, XL.y), make_float2(YL.x, YL.y), make_float2(ZL.x, ZL.y),
                                                make_float2(M.x, M.y), make_float2(VX.x, VX.y), make_float2(VY.x, VY.y),
-                                               make_float2(VZ.x, VZ.y), make_int2(ID.x, ID.y), IP[k], eps2, a[k], tmin[k]);
+                                               make_float2(VZ.x, VZ.y), make_int2(ID.x, ID.y), 2, IP[k], eps2, a[k], tmin[k]);
                     pgb::g6_jpair<true, false>(make_float2(XH.z, XH.w), make_float2(YH.z, YH.w), make_float2(ZH.z, ZH.w),
                                                make_float2(XL.z, XL.w), make_float2(YL.z, YL.w), make_float2(ZL.z, ZL.w),
                                                make_float2(M.z, M.w), make_float2(VX.z, VX.w), make_float2(VY.z, VY.w),
-                                               make_float2(VZ.z, VZ.w), make_int2(ID.z, ID.w), IP[k], eps2, a[k], tmin[k]);
+                                               make_float2(VZ.z, VZ.w), make_int2(ID.z, ID.w), 2, IP[k], eps2, a[k], tmin[k]);
                 }
             }
         }
