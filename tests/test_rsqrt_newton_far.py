@@ -50,3 +50,24 @@ def test_g5_ragged_tiles(kind, cfg):
         # a dozen FP32 operations a pair term, as in test_g5_slots.py
         np.testing.assert_allclose(out[si, :3], ao, rtol=2e-6, atol=2e-6 * np.abs(ao).max(), err_msg=f"nj {nj[q]}")
         np.testing.assert_allclose(np.abs(out[si, 3]), po, rtol=2e-6, err_msg=f"nj {nj[q]}")
+
+
+@pytest.mark.parametrize("n", [2, 3, 5, 257, 513, 771])
+def test_integrator_odd_chunks(n):
+    """The step kernel's j-chunks of an odd number of particles: start-up forces of n particles."""
+    g6 = pgb.ffi.G6("libpg6_newton.so")
+    g6.L.g6_open(0)
+    rng = W.Rng(93 + n)
+    x = _points(rng, n)
+    v = rng.uniform(3 * n).reshape(-1, 3) - 0.5
+    m = np.full(n, MASS)
+    H = pgb.ffi.Hermite(g6, m, x, v, EPS2, 0.2, 0.01, 0.125)
+    try:
+        s = H.get()
+    finally:
+        H.close()
+    ref = O.g6_force(x, v.astype(np.float32).astype(np.float64), np.arange(n, dtype=np.int32), np.float32(EPS2), x,
+                     v.astype(np.float32).astype(np.float64), m, np.arange(n, dtype=np.int32))
+    # FP32 pair terms; the tolerances of test_g6_quad_nn.py (acc 2e-6, the cancelling jerk 1e-5 of the largest)
+    np.testing.assert_allclose(s["acc"], ref["acc"], rtol=2e-6, atol=2e-6 * np.abs(ref["acc"]).max())
+    np.testing.assert_allclose(s["jrk"], ref["jrk"], rtol=1e-5, atol=1e-5 * np.abs(ref["jrk"]).max())
