@@ -1058,7 +1058,7 @@ __device__ __forceinline__ void g6_task(const G6Args& A, const Task& T, unsigned
                 }
             }
         };
-        if (USE_JP ? (self_tile || nt4 != NJ) : self_tile) run_tile(BoolC<true>{});
+        if (USE_JP ? (self_tile || nt != NJ) : self_tile) run_tile(BoolC<true>{});
         else run_tile(BoolC<false>{});
 
         if constexpr (TILEMIN) {
