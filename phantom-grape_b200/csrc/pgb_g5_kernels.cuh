@@ -631,8 +631,10 @@ __global__ void __launch_bounds__(NT) g5_kernel(G5Args A) {
 // particles 2906 -> 2282 us (1955 Gint/s; 12 FMA operations, 4 integer ones and a table look-up of
 // 2.2 shared wavefronts a pair: FMA heavy half 65 %, shared wavefronts 70 %, issue 65 % busy).
 // A j-tile is G5S_NJ records as field arrays; lane l takes the tile's j-quads l, l + 4, ....  The
-// records of a last, partial quad are taken one by one (padded with massless records far away
-// instead, the padding's overflowed r^2 made its terms NaN with the Newton-refined rsqrt).
+// tile is padded to a multiple of 4 with massless records far away (G5S_FAR), which add exact
+// zeros to any finite sum: where r^2 overflows, 1/r is 0.  The Newton-refined rsqrt of an overflowed
+// r^2 is NaN, so with it the records of a last, partial quad are taken one by one instead
+// (G5S_TAIL; in the default build that made launches of 5 to 15 us 0.6 to 1 us longer).
 // FP32 sums cover a tile (32 terms a lane half and i at most), then go
 // into the FP64 sums; the lanes' sums are added in lane order at the end of the task.
 constexpr int G5S_NT = 64, G5S_SLOTS = 16, G5S_LANES = 4, G5S_IPT = 4;
@@ -641,6 +643,13 @@ constexpr int G5S_NJ = 256;   // records a tile: 64 a lane between two folds int
 // registers, which reload the j fields per pair, 3639), point masses and the table 10 (95 registers)
 template <int KIND>
 constexpr int g5s_min_ctas() { return KIND == G5_QUAD ? 5 : 10; }
+
+constexpr float G5S_FAR = 1e18f;   // its square times three is finite
+#ifdef PGB_RSQRT_NEWTON
+constexpr bool G5S_TAIL = true;
+#else
+constexpr bool G5S_TAIL = false;
+#endif
 
 template <int KIND>
 struct G5STile {
@@ -684,14 +693,14 @@ __device__ __forceinline__ void g5_slots_task(const G5Args& A, const Task& T, G5
     };
     load_idx(0);
     for (int jt = 0; jt < T.nj; jt += NJ) {
-        const int nt = min(NJ, T.nj - jt), whole = nt >> 2;
+        const int nt = min(NJ, T.nj - jt), nq = G5S_TAIL ? nt >> 2 : (nt + 3) >> 2;
         float4 J[R];
         float4 Q0[R], Q1[R];
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const int q = tid + r * G5S_NT;
-            // (a value for every thread: without it ptxas spills 200 to 480 bytes)
-            J[r] = Q0[r] = Q1[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+            J[r] = make_float4(G5S_FAR, G5S_FAR, G5S_FAR, 0.f);
+            Q0[r] = Q1[r] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (q < nt) {
                 const int jj = jn[r];
                 J[r] = A.jpos[jj];
@@ -706,7 +715,7 @@ __device__ __forceinline__ void g5_slots_task(const G5Args& A, const Task& T, G5
 #pragma unroll
         for (int r = 0; r < R; r++) {
             const int q = tid + r * G5S_NT;
-            if (q < nt) {
+            if (q < (G5S_TAIL ? nt : 4 * nq)) {
                 float(*f)[NJ] = sh.t.f;
                 f[0][q] = J[r].x;
                 f[1][q] = J[r].y;
@@ -744,7 +753,7 @@ __device__ __forceinline__ void g5_slots_task(const G5Args& A, const Task& T, G5
             }
         };
 #pragma unroll 1
-        for (int jq = lane; jq < whole; jq += G5S_LANES) {
+        for (int jq = lane; jq < nq; jq += G5S_LANES) {
             float4 v[4 + G5STile<KIND>::NQ];
 #pragma unroll
             for (int c = 0; c < 4 + G5STile<KIND>::NQ; c++) v[c] = *reinterpret_cast<const float4*>(&sh.t.f[c][4 * jq]);
@@ -758,9 +767,9 @@ __device__ __forceinline__ void g5_slots_task(const G5Args& A, const Task& T, G5
                 for (int k = 0; k < IPT; k++) add(k, w, a[k]);
             }
         }
-        if (lane == whole % G5S_LANES) {
+        if (G5S_TAIL && lane == nq % G5S_LANES) {
 #pragma unroll 1
-            for (int j = 4 * whole; j < nt; j++) {
+            for (int j = 4 * nq; j < nt; j++) {
                 float2 w[4 + G5STile<KIND>::NQ];
 #pragma unroll
                 for (int c = 0; c < 4 + G5STile<KIND>::NQ; c++) w[c] = make_float2(sh.t.f[c][j], sh.t.f[c][j]);
