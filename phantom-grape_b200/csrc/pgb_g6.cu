@@ -389,7 +389,8 @@ long long plan_items(std::vector<Task>& tasks, std::vector<Group>& groups, int& 
             if (jc < 128) jc = 128;
             if (jc * maxch < nj) jc = (nj + maxch - 1) / maxch;
         }
-        if (jc > nj) jc = nj > 0 ? nj : 1;
+        if (jc > nj) jc = nj;
+        if (jc < 1) jc = 1;   // no j-records: one empty task
         rows += plan_item(tasks, groups, items[4 * k], ni, items[4 * k + 2], nj, itile, (int)jc, rows,
                           align);
         inter += (long long)ni * nj;
