@@ -58,6 +58,9 @@ inline bool abort_enabled(ErrorSlot& e) {
 }
 
 inline void raise(ErrorSlot& e, const char* lib, int code, const char* fmt, ...) {
+    // a call that failed has left its error for the next cudaGetLastError(): a later launch's check would
+    // report it again, for a launch that did not fail
+    if (code == PGB_ERR_CUDA) cudaGetLastError();
     char buf[512];
     va_list ap;
     va_start(ap, fmt);
