@@ -1053,8 +1053,26 @@ bool read_note(pgbt_tree* T, const Note& note, int& v) {
     return false;
 }
 
+// The events that time a build; and, however it ends, nothing reads the caller's arrays any more when
+// it returns: a build that fails half-way waits for both uploads.
+struct BuildScope {
+    pgbt_tree* T;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    bool finished = false;
+    ~BuildScope() {
+        if (!finished) {
+            if (T->s) cudaStreamSynchronize(T->s);
+            if (T->s_up) cudaStreamSynchronize(T->s_up);
+        }
+        if (e0) cudaEventDestroy(e0);
+        if (e1) cudaEventDestroy(e1);
+    }
+};
+
 bool build(pgbt_tree* T, const double* xh, const double* mh) {
     const int n = T->n;
+    BuildScope scope{T};
+    cudaEvent_t &e0 = scope.e0, &e1 = scope.e1;
     cudaStream_t s = T->s;
     std::vector<DevBuf<int>>& stmp = T->stmp;
     std::vector<DevBuf<long long>>& ltmp = T->ltmp;
@@ -1070,7 +1088,6 @@ bool build(pgbt_tree* T, const double* xh, const double* mh) {
     PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(T->m.p, mh, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, T->s_up),
                 return false);
     PGB_CUDA_OR(g_err, LIB, cudaEventRecord(T->up[1], T->s_up), return false);
-    cudaEvent_t e0, e1;
     PGB_CUDA_OR(g_err, LIB, cudaEventCreate(&e0), return false);
     PGB_CUDA_OR(g_err, LIB, cudaEventCreate(&e1), return false);
     PGB_CUDA_OR(g_err, LIB, cudaEventRecord(e0, s), return false);
@@ -1260,8 +1277,7 @@ bool build(pgbt_tree* T, const double* xh, const double* mh) {
     PGB_CUDA_OR(g_err, LIB, cudaEventRecord(e1, s), return false);
     PGB_CUDA_OR(g_err, LIB, cudaEventSynchronize(e1), return false);
     cudaEventElapsedTime(&T->build_ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    scope.finished = true;
     return true;
 }
 
