@@ -944,11 +944,16 @@ bool ensure_device() {
 
 // log2 of the list units a group: more of them shorten the longest walk (whose length goes as
 // theta^-3), fewer test fewer ancestors (at a unit's start; ng 2^ulog times) and keep fewer counts (32
-// bytes a unit).  Measured, count + fill (us) with 64 / 128 / 256 / 512 units, and with the 64 cells two
+// bytes a unit: above 65536 groups no more than 2 KB a group, as the 64 cells took).  Measured, count + fill
+// (us) with 64 / 128 / 256 / 512 units, and with the 64 cells two
 // levels below the root: 2^20 Hernquist particles in 13880 groups, theta 0.5: 1715 / 1507 / 1213 / 1502
 // (2927); 2^22 in 55032: 3875 / 3799 / 4275 / 5507 (4710); 50000 in 1378: 275 / 165 / 124 / 144 (959); 2^18
-// in 13883, theta 0.75: 454 / 400 / 495 / 740 (684).
-int list_unit_log(int ng, double theta) { return ng <= 32768 && (double)ng * theta * theta * theta <= 2500.0 ? 8 : 7; }
+// in 13883, theta 0.75: 454 / 400 / 495 / 740 (684).  A rebuild (ms) with 64 / 128, theta
+// 0.75: 2^22 in 110787 7.8 / 8.5, in 221477 9.7 / 11.4, 2^23 in 442052 18.8 / 24.4.
+int list_unit_log(int ng, double theta) {
+    if (ng > 65536) return 6;
+    return ng <= 32768 && (double)ng * theta * theta * theta <= 2500.0 ? 8 : 7;
+}
 
 inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
