@@ -192,10 +192,21 @@ int occupancy_of(int kind, int cfg) {
 // 26.5 / 37.2 / 98.8, 4096^2 21.7 / 35.1 / 35.3, 8000^2 46.0 / 47.5 / 51.5, 16384^2 146 / 133 / 148,
 // 65536^2 2022 / 1914 / 2162; a tree of 2^16 particles 55 (points) and 195 (cells) against 370 and
 // 1636 with 128x2, 310-particle TreePM groups 2282 against 5319 with 256x2.
-constexpr long long G5_LARGE_NI = 12288;
-int pick_cfg(int kind, long long ni_max) {
+// Items of few j give the slot kernel's tasks too little to do for what starting and ending one costs;
+// such items, unless they are few i too, run 128x1 (us, 64x1 / 128x1 / the
+// default before the slot kernel): quad 262144 x 4 16.6 / 8.4 / 8.4, x 32 20.7 / 16.6 / 18.1, 1000 items of
+// 300 x 10 18.7 / 12.5 / 12.5, 64 x 4 6.3 / 4.6 / 4.9; table 262144 x 64 22.8 / 20.7 / 20.7; symmetric 262144 x
+// 16 12.5 / 8.4 / 10.5, 20000 cell items of 1 x 1 41 / 25 / 31.  The other way: quad 65536 x 64 10.7 / 11.4 / 12.5, 20000 items of 8 x 16 41 / 70 / 117.
+constexpr long long G5_LARGE_NI = 12288, G5_FEW_NJ = 16, G5_FEW_NJ_MANY = 64, G5_MANY_NI = 1 << 17;
+int forced_cfg(int kind) {
     static int forced = env_int("PGB_G5_CFG", -1, -1, G5_NCFG - 1);
-    if (forced >= 0 && cfg_valid(kind, forced)) return forced;
+    return forced >= 0 && cfg_valid(kind, forced) ? forced : -1;
+}
+// ni_max, nj_max: the largest item's; ni_sum: all items' i.  (nj_max 0: nothing known yet.)
+int pick_cfg(int kind, long long ni_max, long long nj_max, long long ni_sum) {
+    if (forced_cfg(kind) >= 0) return forced_cfg(kind);
+    const long long few = ni_max < 64 ? 2 : ni_sum > G5_MANY_NI ? G5_FEW_NJ_MANY : G5_FEW_NJ;
+    if (nj_max > 0 && nj_max <= few) return G5C_128x1;
     return kind == G5_NEWTON && ni_max > G5_LARGE_NI ? G5C_1024x1J : G5C_64x1;
 }
 
@@ -520,7 +531,14 @@ bool flush_c(Dev& d) {
 // one copies them (half the bytes) and waits for the stream.  Measured (us a call, copied / words): 250 x 250
 // 52 / 40, 999 x 999 53 / 48, 2000 63 / 58, 4096 99 / 87.
 constexpr int G5_WORDS_NI = 4096;
-bool sends_words(int kind, int ni) { return ni <= G5_WORDS_NI && G5C_NT[pick_cfg(kind, ni)] == G5S_NT; }
+bool sends_words(int kind, int ni) {
+    return ni <= G5_WORDS_NI && (forced_cfg(kind) < 0 || G5C_NT[forced_cfg(kind)] == G5S_NT);
+}
+// A call's configuration: one that sends words runs the kernel that can.
+int call_cfg(int kind, int ni, int nj, bool words) {
+    if (forced_cfg(kind) >= 0) return forced_cfg(kind);
+    return words ? G5C_64x1 : pick_cfg(kind, ni, nj, ni);
+}
 
 // Launch `kind` for ni i-records, which fill(dst) writes, against this devid's j-memory (nbody records)
 // or cell memory (ncell cells).  The results land in d.outh after the stream synchronises, or, with
@@ -549,7 +567,7 @@ bool compute(Dev& d, int kind, int ni, Fill fill, bool words) {
     }
     std::vector<Task> tasks;
     std::vector<Group> groups;
-    const int cfg = pick_cfg(kind, ni);
+    const int cfg = call_cfg(kind, ni, nj, words);
     const int itile = cfg_itile(cfg);
     int slots = sm_count(g_device) * occupancy_of(kind, cfg);
     long long itiles = (ni + itile - 1) / itile;
@@ -1162,10 +1180,14 @@ PGB_EXPORT int pgb5_plan_create(pgb5_plan** out, int kind, int nitem, const int*
     P->kind = kind;
     P->items.assign(items, items + 4 * (size_t)nitem);
     P->shape_key = shape_key(kind, nitem, items);
-    long long nimax = 0;
-    for (int k = 0; k < nitem; k++) nimax = std::max<long long>(nimax, items[4 * k + 1]);
+    long long nimax = 0, njmax = 0, nisum = 0;
+    for (int k = 0; k < nitem; k++) {
+        nimax = std::max<long long>(nimax, items[4 * k + 1]);
+        njmax = std::max<long long>(njmax, items[4 * k + 3]);
+        nisum += items[4 * k + 1];
+    }
     const int tuned = tuned_cfg(P->shape_key);
-    P->cfg = tuned >= 0 ? tuned : pick_cfg(kind, nimax);
+    P->cfg = tuned >= 0 ? tuned : pick_cfg(kind, nimax, njmax, nisum);
     plan_items(P);
     cudaStream_t s = nullptr;
     bool ok = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
