@@ -528,11 +528,14 @@ bool flush_c(Dev& d) {
 }
 
 // A call of at most this many i sends its results as words that the host takes as they arrive; a larger
-// one copies them (half the bytes) and waits for the stream.  Measured (us a call, copied / words): 250 x 250
-// 52 / 40, 999 x 999 53 / 48, 2000 63 / 58, 4096 99 / 87.
+// one copies them (half the bytes) and waits for the stream.  The words are written while the pairs
+// are summed, which hides them from about a j for 16 i on; a call of more i for its j copies them
+// too.  Measured (us a call, copied / words): 250 x 250 52 / 40, 999 x 999 53 / 48, 2000 63 / 58, 4096 99 / 87;
+// 500 x 1 36 / 40, 500 x 30 30 / 28, 1000 x 30 32 / 34, 1000 x 100 39 / 37, 2000 x 100 46 / 82, 2000 x 300 47 / 47,
+// 4096 x 100 59 / 73, 4096 x 300 63 / 54.
 constexpr int G5_WORDS_NI = 4096;
-bool sends_words(int kind, int ni) {
-    return ni <= G5_WORDS_NI && (forced_cfg(kind) < 0 || G5C_NT[forced_cfg(kind)] == G5S_NT);
+bool sends_words(int kind, int ni, int nj) {
+    return ni <= G5_WORDS_NI && ni <= 256 + 16LL * nj && (forced_cfg(kind) < 0 || G5C_NT[forced_cfg(kind)] == G5S_NT);
 }
 // A call's configuration: one that sends words runs the kernel that can.
 int call_cfg(int kind, int ni, int nj, bool words) {
@@ -710,7 +713,7 @@ void calc_impl(int devid, int kind, const double (*x)[3], const double* eps2, do
     std::lock_guard<std::mutex> g(dj->mu);
     if (!quiesce(*dj)) return;
     const float e_all = (float)(g_eps * g_eps);
-    const bool words = sends_words(kind, ni);
+    const bool words = sends_words(kind, ni, kind == G5_QUAD ? dj->ncell : dj->nbody);
     auto fill = [&](float4* r) {
         for (int i = 0; i < ni; i++) r[i] = make_i(x[i], eps2 ? (float)eps2[i] : e_all);
     };
