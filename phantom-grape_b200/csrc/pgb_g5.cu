@@ -611,7 +611,9 @@ void write_out(const double4* o, int ni, double (*a)[3], double* p) {
 }
 
 // The results of a call that sends words, as they arrive: a bounded spin, then the stream
-// synchronisation that reports a failed launch.
+// synchronisation that reports a failed launch.  They also go where g5_get_force reads, as a copied
+// call's do: a call is g5_set_xi, g5_run and g5_get_force (phantom_g5.c:276-300), and what its pipelines
+// hold afterwards are its own results.
 bool take_words(Dev& d, int ni, double (*a)[3], double* p) {
     const volatile unsigned long long* w = (const volatile unsigned long long*)d.words.p;
     int i = 0;
@@ -624,6 +626,7 @@ bool take_words(Dev& d, int ni, double (*a)[3], double* p) {
                 const unsigned long long v = hi << 32 | (lo & 0xffffffffull);
                 std::memcpy(&o[c], &v, sizeof v);
             }
+            if (i < d.pending) d.outh.p[i] = make_double4(o[0], o[1], o[2], o[3]);
             write_one(o, i, a, p);
         }
         return true;
