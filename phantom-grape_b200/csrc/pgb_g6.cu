@@ -98,6 +98,7 @@ constexpr int ITILE_MAX = 512;
 struct KernelInfo {
     int occ = 0, tile = 0, itile = 0;
     bool paired = false;    // the j-paired form
+    double task_j = 64.0;   // best_nch's
     double tail = 0.2;      // best_tile_chunk's (the stage-ordered form loses more with few CTAs on an SM:
                             // 65536 x 65536 in 8 chunks 4996 us, in 16 to 19 4664)
     bool resolve = false;   // leaves the nearest-neighbour lookups of split i-tiles to g6_resolve_kernel
@@ -112,6 +113,7 @@ void one_kernel(int grid, const G6Args& a, cudaStream_t s, KernelInfo* info) {
         info->tile = g6_tile_j<NT, JL, g6_uses_jp<IPT, FF, NBL, JP>()>();
         info->itile = NT / JL * IPT;
         info->paired = g6_uses_jp<IPT, FF, NBL, JP>();
+        info->task_j = NT == 512 ? 256.0 : 64.0;
         info->tail = JP == 2 ? 0.5 : 0.2;
         info->resolve = NN && !NBL && IPT % 2 == 0 && !g6_quad_min<IPT, FF, NBL, JP>();
         return;
@@ -346,7 +348,7 @@ int pick_batch_cfg(int nitem, const int* items, bool ff) {
 // The chunk length of a single item: the j-paired kernels' whole tiles, else the wave model's.
 long long model_chunk(const KernelInfo& K, long long itiles, int nj, int slots, int maxch) {
     if (K.paired) return best_tile_chunk(itiles, nj, sm_count(g_device), K.tile, maxch, K.tail);
-    const int nch = best_nch(itiles, nj, slots, maxch);
+    const int nch = best_nch(itiles, nj, slots, maxch, K.task_j);
     return (nj + nch - 1) / nch;
 }
 
@@ -732,11 +734,12 @@ bool run_force(int nj, int ni, float eps2, bool nn, bool nbl) {
     if (ni <= G6_SMALL_MAXI && nj > 0) return run_small(nj, ni, eps2, nn, nbl);
     const bool ff = dx_ff();
     const int cfg = pick_cfg(ni, nj, ff, nbl);
-    const int itile = kernel_info(cfg, ff, nn, nbl).itile;
-    const int slots = sm_count(g_device) * occupancy(cfg, ff, nn, nbl);
+    const KernelInfo K = kernel_info(cfg, ff, nn, nbl);
+    const int itile = K.itile;
+    const int slots = sm_count(g_device) * K.occ;
     static const int maxch = env_int("PGB_G6_MAXCHUNKS", 512, 1, 4096);
     const int itiles = (ni + itile - 1) / itile;
-    int nch = best_nch(itiles, nj, slots, maxch);
+    int nch = best_nch(itiles, nj, slots, maxch, K.paired ? 256.0 : K.task_j);
     if (nch > nj) nch = nj > 0 ? nj : 1;
     const int rows = nch > 1 ? itiles * nch : 0;
     static const std::vector<Task> no_tasks;
