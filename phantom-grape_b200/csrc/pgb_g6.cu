@@ -1608,15 +1608,15 @@ namespace {
 std::mutex g_na_mu;
 void* g_na_addr[64];  // device address of g6_noalloc_scratch per device (set-up once)
 
-// Regular decomposition of one (ni x nj) item into itiles x nch tasks, written to the scratch
+// Regular decomposition of one (ni x nj) item into itiles x nch tasks of jc j, written to the scratch
 // work list (the layout the force kernel reads from a staged plan).
-__global__ void g6_regular_tasks(Task* tasks, Group* groups, int ni, int nj, int itile, int itiles, int nch) {
+__global__ void g6_regular_tasks(Task* tasks, Group* groups, int ni, int nj, int itile, int itiles, int nch, int jc) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= itiles * nch) return;
     int it = t / nch, c = t % nch;
     int i0 = it * itile;
     int nii = min(itile, ni - i0);
-    int j0 = (int)((long long)c * nj / nch), j1 = (int)((long long)(c + 1) * nj / nch);
+    int j0 = c * jc, j1 = c + 1 < nch ? j0 + jc : nj;
     if (nch == 1) {
         tasks[t] = Task{i0, nii, 0, nj, -1, 0, -1, 0};
         return;
@@ -1671,22 +1671,22 @@ PGB_EXPORT int pgb6_force_noalloc(const void* ipart, int ni, const void* jpred, 
         }
         base = g_na_addr[g_device];
     }
-    // j-chunks per i-tile: about 4 tasks per resident CTA, at least 128 j per chunk, within
-    // the scratch's task and partial-row capacity
-    const int slots = sm_count(g_device) * occupancy(cfg, ff, nn, false);
-    long long nch = (4LL * slots + itiles - 1) / itiles;
-    nch = std::min<long long>(nch, std::max<long long>(1, nj / 128));
-    nch = std::min<long long>(nch, 512);
-    nch = std::min<long long>(nch, NOALLOC_MAX_TASKS / itiles);
-    nch = std::min<long long>(nch, (long long)(NOALLOC_MAX_PART / ((size_t)itiles * itile)));
-    if (nch < 1) nch = 1;
+    // j-chunks per i-tile: a single-item plan's (model_chunk), within the scratch's task and
+    // partial-row capacity.  (About four tasks per resident CTA instead: 777 x 65536 201 us, 2048 x 4096 47.)
+    const KernelInfo K = kernel_info(cfg, ff, nn, false);
+    const int slots = sm_count(g_device) * K.occ;
+    long long maxch = std::min<long long>(512, NOALLOC_MAX_TASKS / itiles);
+    maxch = std::min<long long>(maxch, (long long)(NOALLOC_MAX_PART / ((size_t)itiles * itile)));
+    if (maxch < 1) maxch = 1;
+    const long long jc = nj > 0 ? std::min<long long>(nj, model_chunk(K, itiles, nj, slots, (int)maxch)) : 1;
+    const long long nch = nj > 0 ? (nj + jc - 1) / jc : 1;
     const int ntasks = (int)(itiles * nch);
     unsigned char* b = (unsigned char*)base;
     cudaStream_t s = (cudaStream_t)stream;
     // the task counter and the group counters must start at zero
     PGB_CUDA_OR(g_err, LIB, cudaMemsetAsync(b, 0, NA_OFF_TASKS, s), return PGB_ERR_CUDA);
     g6_regular_tasks<<<(ntasks + 255) / 256, 256, 0, s>>>((Task*)(b + NA_OFF_TASKS), (Group*)(b + NA_OFF_GROUPS), ni,
-                                                          nj, itile, (int)itiles, (int)nch);
+                                                          nj, itile, (int)itiles, (int)nch, (int)jc);
     PGB_CUDA_OR(g_err, LIB, cudaGetLastError(), return PGB_ERR_CUDA);
     G6Args a;
     a.ipart = (const G6I*)ipart;
