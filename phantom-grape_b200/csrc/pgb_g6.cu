@@ -89,7 +89,10 @@ bool ensure_device() {
 
 enum Cfg {
     CFG_SMALL = 0, CFG_MED = 1, CFG_LARGE = 2, CFG_128x1 = 3, CFG_128x4 = 4, CFG_256x2 = 5,
-    CFG_128x2J = 6, CFG_256x2J = 7, CFG_128x4J = 8, CFG_128x2JS = 9, NCFG = 10
+    CFG_128x2J = 6, CFG_256x2J = 7, CFG_128x4J = 8, CFG_128x2JS = 9, NCFG = 10,
+    // CFG_MED's form of one i per thread also where the j-paired one applies: a choice of the default rules
+    // and the tuner, not settable and reported as CFG_MED, whose i-tile it has
+    CFG_MED1 = NCFG
 };
 constexpr int ITILE_MAX = 512;
 
@@ -142,6 +145,7 @@ void cfg_kernel(int cfg, int grid, const G6Args& a, cudaStream_t s, KernelInfo* 
     switch (cfg) {
         case CFG_SMALL: one_kernel<512, 1, 8, FF, NN, NBL, 0>(grid, a, s, info); break;
         case CFG_MED: med_kernel<FF, NN, NBL>(grid, a, s, info); break;
+        case CFG_MED1: one_kernel<256, 1, 2, FF, NN, NBL, 0>(grid, a, s, info); break;
         case CFG_128x1: quad_kernel<FF, NN, NBL>(grid, a, s, info); break;
         case CFG_128x4: one_kernel<128, 4, 1, FF, NN, NBL, 0>(grid, a, s, info); break;
         case CFG_256x2: one_kernel<256, 2, 1, FF, NN, NBL, 0>(grid, a, s, info); break;
@@ -168,13 +172,14 @@ void any_kernel(int cfg, bool ff, bool nn, bool nbl, int grid, const G6Args& a, 
 
 KernelInfo kernel_info(int cfg, bool ff, bool nn, bool nbl) {
     static std::mutex mu;
-    static KernelInfo cache[NCFG][8];
+    static KernelInfo cache[NCFG + 1][8];
     std::lock_guard<std::mutex> g(mu);
     KernelInfo& v = cache[cfg][(ff ? 4 : 0) | (nn ? 2 : 0) | (nbl ? 1 : 0)];
     if (!v.occ) any_kernel(cfg, ff, nn, nbl, 0, G6Args{}, nullptr, &v);
     return v;
 }
 int occupancy(int cfg, bool ff, bool nn, bool nbl) { return kernel_info(cfg, ff, nn, nbl).occ; }
+int reported_cfg(int cfg) { return cfg == CFG_MED1 ? (int)CFG_MED : cfg; }
 
 cudaError_t launch_kernel(int cfg, bool ff, bool nn, bool nbl, int grid, const G6Args& a, cudaStream_t s) {
     any_kernel(cfg, ff, nn, nbl, grid, a, s, nullptr);
@@ -311,11 +316,16 @@ bool dx_ff() {
 //   4096 x 16384  140   /  101   /  121    8192 x 16384  244   /  177   /  198   (220)
 //   8192 x 65536  876   /  646   /  632 (749)   16384 x 16384  458 / 329 / 344 (399)
 //   16384 x 65536  1718 / 1260 / 1208 (1457)    65536 x 65536  6754 / 4890 / 4664 (5488)
-int pick_cfg(long long ni, long long nj, bool ff, bool nbl) {
+// Few j: the scalar forms, whose tasks start and end sooner, up to 4096 i against 256 j (CFG_MED1 / MED: 4096 x
+// 32 6.4 / 8.4, x 200 12.5 / 15.0) and for the most i against the fewest j (LARGE / MED: 131072 x 4 10.5 / 15.3,
+// x 32 20 / 19; without neighbours 65536 x 64 12.5 / 14.6).
+int pick_cfg(long long ni, long long nj, bool ff, bool nn, bool nbl) {
     static int forced = env_int("PGB_G6_CFG", -1, -1, NCFG - 1);
     if (forced >= 0) return forced;
     if (ff && !nbl) {
         if (ni <= 3072 && ni * nj <= (ni <= 1024 ? 48LL << 20 : 24LL << 20)) return CFG_SMALL;
+        if (ni <= 4096 && nj <= 256) return CFG_MED1;
+        if (ni >= 32768 && nj <= (nn ? 16 : 64)) return CFG_LARGE;
         return ni * nj < (1LL << 29) ? CFG_MED : CFG_128x2JS;
     }
     if (ni <= 64) return CFG_SMALL;
@@ -323,25 +333,44 @@ int pick_cfg(long long ni, long long nj, bool ff, bool nbl) {
     return CFG_LARGE;
 }
 
-// The same for a batch of several items, by the i count that the average pair sees: MED's smaller
-// i-tiles up to 6000, then CFG_128x1's j-paired form (us, MED / 128x1 / the scalar form that was the
-// default: 40 clusters of 300 to 5000 particles 220 / 234 / 327, 96 of 64 to 2048 110 / 122 / 192, 96 of
-// 256 to 16384 4352 / 4227 / 5136).
-int pick_batch_cfg(int nitem, const int* items, bool ff) {
+// The same for a batch of several items.
+//  * Short work, up to 2^20 pairs of SMALL's 64-i tiles (at least 128 j): SMALL (us, SMALL / MED: 4 items of 16 i x
+//    4096 j 12.5 / 14.6, 64 of 100 x 128 8.4 / 9.5).
+//  * Items of at most 64 i, whose tiles of 128 MED leaves half empty: SMALL where its tasks, one wave of a
+//    few long ones, fill the GPU, that is for many items of many j (256 of 1 i x 1024 j 37 / 55, 64 of 4 x 4096
+//    50 / 59, 96 of 1 x 1024 27 / 29) and for two to four (2 of 48 x 65536 39 / 48, 2 of 64 x 16384 20.7 / 22.8, 4 of 64 x
+//    65536 64 / 69); else MED (8 of 8 x 65536 115 / 99, 2 of 32 x 16384 20.7 / 18.7, 32 of 8 x 1024 18.6 / 14.6, 1024 of 4 x
+//    128 37 / 28).
+//  * Middle work of up to 32 tiles: MED1, whose threads have one i where MED's have two (4 items of 128 x 4096
+//    17.6 / 23.8, 2 of 100 x 16384 24.8 / 29.2, 16 of 128 x 1024 14.4 / 16.6); from 2^25 pairs on MED (4 of 100 x 65536 84 / 79).
+//  * Then by the i count that the average pair sees: MED's smaller i-tiles up to 6000, above that
+//    CFG_128x1's j-paired form (us, MED / 128x1 / the scalar form that was the default: 40 clusters of
+//    300 to 5000 particles 220 / 234 / 327, 96 of 64 to 2048 110 / 122 / 192, 96 of 256 to 16384 4352 / 4227 / 5136).
+int pick_batch_cfg(int nitem, const int* items, bool ff, bool nn) {
     double w = 0.0, wi = 0.0;
-    long long nimax = 0, njmax = 0, total_i = 0;
+    long long nimax = 0, njmax = 0, total_i = 0, tiles = 0, pairs64 = 0, pairs128 = 0;
     for (int k = 0; k < nitem; k++) {
         const long long ni = items[4 * k + 1], nj = items[4 * k + 3];
         nimax = std::max(nimax, ni);
         njmax = std::max(njmax, nj);
         total_i += ni;
+        tiles += (ni + 127) / 128;
+        pairs64 += (ni + 63) / 64 * 64 * nj;
+        pairs128 += (ni + 127) / 128 * 128 * nj;
         w += (double)ni * (double)nj;
         wi += (double)ni * (double)nj * (double)ni;
     }
-    if (nitem == 1) return pick_cfg(nimax, njmax, ff, false);
-    if (!ff) return pick_cfg(std::max(nimax, total_i / 4), njmax, ff, false);
+    if (nitem == 1) return pick_cfg(nimax, njmax, ff, nn, false);
+    if (!ff) return pick_cfg(std::max(nimax, total_i / 4), njmax, ff, nn, false);
     static int forced = env_int("PGB_G6_CFG", -1, -1, NCFG - 1);
     if (forced >= 0) return forced;
+    if (pairs64 <= (1 << 20) && njmax >= 128) return CFG_SMALL;
+    if (nimax <= 64) {
+        const bool many = nitem >= 48 && njmax >= 512 && pairs64 >= (5 << 20);
+        const bool few = (nitem <= 4 && nimax > 32) || (nitem <= 3 && njmax > 32768);
+        return many || few ? CFG_SMALL : CFG_MED;
+    }
+    if (tiles <= 32 && pairs128 < (1 << 25)) return CFG_MED1;
     return wi <= 6000.0 * w ? CFG_MED : CFG_128x1;
 }
 
@@ -733,7 +762,7 @@ bool run_force(int nj, int ni, float eps2, bool nn, bool nbl) {
     }
     if (ni <= G6_SMALL_MAXI && nj > 0) return run_small(nj, ni, eps2, nn, nbl);
     const bool ff = dx_ff();
-    const int cfg = pick_cfg(ni, nj, ff, nbl);
+    const int cfg = pick_cfg(ni, nj, ff, nn, nbl);
     const KernelInfo K = kernel_info(cfg, ff, nn, nbl);
     const int itile = K.itile;
     const int slots = sm_count(g_device) * K.occ;
@@ -1230,7 +1259,7 @@ PGB_EXPORT int pgb6_plan_create(pgb6_plan** out, int nitem, const int* items, in
     P->jend = items_jend(nitem, items);
     P->shape_key = shape_key(nitem, items, P->ff, P->nn);
     const Tuned tuned = tuned_cfg(P->shape_key);
-    P->cfg = tuned.cfg >= 0 ? tuned.cfg : pick_batch_cfg(nitem, items, P->ff);
+    P->cfg = tuned.cfg >= 0 ? tuned.cfg : pick_batch_cfg(nitem, items, P->ff, P->nn);
     P->nch = tuned.cfg >= 0 ? tuned.nch : 0;
     P->interactions = plan_items(P->tasks, P->groups, P->rows, nitem, items, P->cfg, P->ff, P->nn, false, P->nch);
     cudaStream_t s = nullptr;
@@ -1250,7 +1279,7 @@ PGB_EXPORT int pgb6_plan_create(pgb6_plan** out, int nitem, const int* items, in
 
 PGB_EXPORT long long pgb6_plan_interactions(const pgb6_plan* P) { return P ? P->interactions : 0; }
 PGB_EXPORT int pgb6_plan_tasks(const pgb6_plan* P) { return P ? (int)P->tasks.size() : 0; }
-PGB_EXPORT int pgb6_plan_config(const pgb6_plan* P) { return P ? P->cfg : -1; }
+PGB_EXPORT int pgb6_plan_config(const pgb6_plan* P) { return P ? reported_cfg(P->cfg) : -1; }
 // j-chunks per i-tile of a one-item plan (1: the j-range unsplit); 0 for plans of several items.
 PGB_EXPORT int pgb6_plan_chunks(const pgb6_plan* P) {
     if (!P || P->items.size() != 4 || P->tasks.empty()) return 0;
@@ -1414,7 +1443,7 @@ PGB_EXPORT int pgb6_plan_tune(pgb6_plan* P, const void* ipart, const void* jpred
         return true;
     };
     std::vector<std::pair<float, int>> by_cfg;
-    for (int cfg = 0; cfg < NCFG; cfg++) {
+    for (int cfg = 0; cfg < (P->ff ? NCFG + 1 : NCFG); cfg++) {   // CFG_MED1 is CFG_MED with FP64 positions
         float t;
         if (!time_plan(cfg, 0, &t)) break;
         by_cfg.emplace_back(t, cfg);
@@ -1463,7 +1492,7 @@ PGB_EXPORT int pgb6_plan_tune(pgb6_plan* P, const void* ipart, const void* jpred
     PGB_CUDA_OR(g_err, LIB, cudaStreamSynchronize(s), return -1);
     set_tuned(P->shape_key, best);
     if (best_ms) *best_ms = best_t;
-    return best.cfg;
+    return reported_cfg(best.cfg);
 }
 
 PGB_EXPORT void pgb6_plan_destroy(pgb6_plan* P) {
@@ -1640,7 +1669,7 @@ PGB_EXPORT int pgb6_force_noalloc(const void* ipart, int ni, const void* jpred, 
     if (ni == 0) return PGB_OK;
     if (!ensure_device()) return PGB_ERR_NOGPU;
     const bool nn = (flags & PGB6_NN) != 0, ff = (flags & PGB6_POS_F64) == 0;
-    int cfg = pick_cfg(ni, nj, ff, false);
+    int cfg = pick_cfg(ni, nj, ff, nn, false);
     int itile = kernel_info(cfg, ff, nn, false).itile;
     if (ni > (long long)NOALLOC_MAX_ITILES * itile) {   // too many small tiles: the 256-particle tile
         cfg = ff ? CFG_128x2JS : CFG_LARGE;
