@@ -1764,16 +1764,24 @@ namespace {
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
-// Co-resident CTAs of the persistent kernel (its cooperative grid).
+const void* hm_kernel(bool ff, bool start) {
+    if (start) return ff ? (const void*)hm_run_kernel<true, true> : (const void*)hm_run_kernel<false, true>;
+    return ff ? (const void*)hm_run_kernel<true, false> : (const void*)hm_run_kernel<false, false>;
+}
+
+// Co-resident CTAs of the persistent kernel (its cooperative grid, the same for both instances).
 int hm_grid(bool ff) {
     static int cache[2] = {0, 0};
     int& g = cache[ff ? 1 : 0];
     if (!g) {
-        int per = 0;
-        cudaError_t e = ff ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, hm_run_kernel<true>, HM_NT, 0)
-                           : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, hm_run_kernel<false>, HM_NT, 0);
-        if (e != cudaSuccess || per < 1) per = 1;
-        g = per * sm_count(g_device);
+        int least = 0;
+        for (bool start : {false, true}) {
+            int per = 0;
+            const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, hm_kernel(ff, start), HM_NT, 0);
+            if (e != cudaSuccess || per < 1) per = 1;
+            least = least ? std::min(least, per) : per;
+        }
+        g = least * sm_count(g_device);
     }
     return g;
 }
@@ -1889,7 +1897,7 @@ bool hm_launch(pgb6_hermite* H, bool startup, double tend, int max_steps) {
     R.nch1 = std::min(H->grid, std::max(1, H->n / minj));
     R.dtinv = 1.0 / H->dtmax;
     void* args[] = {&R};
-    const void* fn = H->ff ? (const void*)hm_run_kernel<true> : (const void*)hm_run_kernel<false>;
+    const void* fn = hm_kernel(H->ff, startup && H->n > HM_SMALL);
     PGB_CUDA_OR(g_err, LIB, cudaLaunchCooperativeKernel(fn, dim3(H->grid), dim3(HM_NT), args, 0, H->s),
                 return false);
     return true;
