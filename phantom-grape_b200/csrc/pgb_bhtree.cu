@@ -32,7 +32,7 @@
 // prefix sum, and a scatter kernel places each particle at child start + tile offset + its rank
 // among the tile's particles of the same octant (warp ballots) -- a stable partition, as the
 // host's counting sort.  Pre-order numbers follow from subtree sizes; sizes and moments are
-// made bottom-up in one launch each; lists by 256 or 128 threads per group (one per equal range of
+// made bottom-up in one launch each; lists by 256, 128 or 64 threads per group (one per equal range of
 // pre-order nodes, walked without a stack), a counting pass, a prefix sum and a filling pass.
 #include <chrono>
 
@@ -1199,7 +1199,6 @@ bool build(pgbt_tree* T, const double* xh, const double* mh) {
         if (nnew == 0) break;
     }
     const int nn = lvl.back();
-    const int nlev = (int)lvl.size() - 1;
     T->nn = nn;
     Nodes N = bfs(T);
 
@@ -1394,7 +1393,8 @@ PGB_EXPORT int pgbt_ngroups(const pgbt_tree* T) { return T ? T->ng : 0; }
 PGB_EXPORT int pgbt_nnodes(const pgbt_tree* T) { return T ? T->nn : 0; }
 PGB_EXPORT long long pgbt_np(const pgbt_tree* T) { return T ? T->np : 0; }
 PGB_EXPORT long long pgbt_nc(const pgbt_tree* T) { return T ? T->nc : 0; }
-// device time of the build (ms, CUDA events from the first kernel to the records)
+// device time of the build (ms, CUDA events from the first kernel to the records, so that what is left of the
+// masses' upload beside the partition counts)
 PGB_EXPORT float pgbt_build_ms(const pgbt_tree* T) { return T ? T->build_ms : 0.f; }
 
 namespace {

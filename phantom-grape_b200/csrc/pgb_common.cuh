@@ -179,7 +179,7 @@ struct Group {
 // persistent CTAs run ceil(itiles*nch/slots) waves of tasks of nj/nch pairs per i, each of which
 // costs `task_j` j more than its pairs (its start, lane sums and partial row; 2086 i x 2134 j on the
 // 512-thread Hermite CTAs: 13 chunks, three waves, 24.9 us, 4 chunks, one wave, 17.4; FP64 positions on the
-// 256-thread ones: 4096 x 65536 in 13 chunks 496, 27 or 37 451, 4096 x 4096 in 13 44, 27 52).  Chunks hold at
+// 256-thread ones: 4096 x 65536 in 13 chunks 496, 27 464, 37 451, 4096 x 4096 in 13 44, 27 52).  Chunks hold at
 // least `minj` j and there are at most `maxch` of them.
 inline int best_nch(long long itiles, long long nj, long long slots, int maxch, double task_j = 256.0, int minj = 128) {
     long long hi = nj / minj;

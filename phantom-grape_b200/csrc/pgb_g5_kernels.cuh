@@ -203,8 +203,7 @@ __device__ __forceinline__ void g5_interact(const float4* sj, int j, float xi, f
 
 __device__ __forceinline__ float& lane_of(float2& v, int k) { return k ? v.y : v.x; }
 
-// Two i-particles of a thread (configurations with IPT >= 2, and the 64-thread CTAs' full
-// tiles) against one j record: the per-i chains exactly as g5_interact / g5_table_pair, the
+// Two i-particles of a thread (configurations with IPT >= 2) against one j record: the per-i chains exactly as g5_interact / g5_table_pair, the
 // accumulations of the two i issued as paired FP32 instructions (FFMA2 / FADD2, each lane rounded
 // as the scalar instruction: results bit-identical to two g5_interact calls), except the
 // quadrupole kind's, whose sums stay scalar (g5_quad_pair per i: its many other FMAs already

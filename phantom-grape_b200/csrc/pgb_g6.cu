@@ -1859,7 +1859,7 @@ bool hm_alloc(pgb6_hermite* H) {
     return true;
 }
 
-// Wait for the stream and read the device clock; a barrier that gave up is an error.
+// Wait for the stream and read the device clock; a wait that gave up is an error.
 bool hm_sync_clock(pgb6_hermite* H) {
     PGB_CUDA_OR(g_err, LIB, cudaMemcpyAsync(&H->clk, H->W.clk, sizeof(HmClock), cudaMemcpyDeviceToHost, H->s),
                 return false);
@@ -2001,11 +2001,11 @@ PGB_EXPORT int pgb6_hermite_advance(pgb6_hermite* H, double tend, long long* pst
 
 PGB_EXPORT double pgb6_hermite_time(pgb6_hermite* H) { return H ? H->clk.time : 0.0; }
 
-// The limit, in SM cycles, of every wait of the step kernel (grid barriers, segment and task
-// flags); cycles <= 0 restores the default (about a second).  A wait that runs out sets the
-// integrator's error word: every CTA returns at its next wait, the call reports PGB_ERR_DEVICE
-// and the integrator is unusable afterwards (its barrier state is no longer consistent).  For
-// fault-handling tests; a production run keeps the default.
+// The limit, in SM cycles, of every wait of the step kernel (segment records and their
+// acknowledgements, chunk sums, segment and task flags); cycles <= 0 restores the default (about a
+// second).  A wait that runs out sets the integrator's error word: every CTA returns at its next wait,
+// the call reports PGB_ERR_DEVICE and the integrator is unusable afterwards (its records and flags no longer
+// agree).  For fault-handling tests; a production run keeps the default.
 PGB_EXPORT int pgb6_hermite_set_wait_limit(pgb6_hermite* H, long long cycles) {
     if (!H) {
         raise(g_err, LIB, PGB_ERR_ARG, "pgb6_hermite_set_wait_limit: null integrator");
