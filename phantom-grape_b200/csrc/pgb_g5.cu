@@ -616,6 +616,7 @@ void write_out(const double4* o, int ni, double (*a)[3], double* p) {
 // hold afterwards are its own results.
 bool take_words(Dev& d, int ni, double (*a)[3], double* p) {
     const volatile unsigned long long* w = (const volatile unsigned long long*)d.words.p;
+    const int keep = std::min(ni, d.pending);
     int i = 0;
     auto take = [&] {
         for (; i < ni; i++) {
@@ -626,7 +627,7 @@ bool take_words(Dev& d, int ni, double (*a)[3], double* p) {
                 const unsigned long long v = hi << 32 | (lo & 0xffffffffull);
                 std::memcpy(&o[c], &v, sizeof v);
             }
-            if (i < d.pending) d.outh.p[i] = make_double4(o[0], o[1], o[2], o[3]);
+            if (i < keep) d.outh.p[i] = make_double4(o[0], o[1], o[2], o[3]);
             write_one(o, i, a, p);
         }
         return true;
