@@ -1443,7 +1443,9 @@ PGB_EXPORT int pgb6_plan_tune(pgb6_plan* P, const void* ipart, const void* jpred
         return true;
     };
     std::vector<std::pair<float, int>> by_cfg;
-    for (int cfg = 0; cfg < (P->ff ? NCFG + 1 : NCFG); cfg++) {   // CFG_MED1 is CFG_MED with FP64 positions
+    // CFG_MED1 is CFG_MED with FP64 positions, and has not been the fastest above 2^25 pairs
+    const int ncfg = P->ff && P->interactions < (1LL << 26) ? NCFG + 1 : NCFG;
+    for (int cfg = 0; cfg < ncfg; cfg++) {
         float t;
         if (!time_plan(cfg, 0, &t)) break;
         by_cfg.emplace_back(t, cfg);
